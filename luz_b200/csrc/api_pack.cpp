@@ -93,6 +93,7 @@ int luz_pack_array(const luz_scene_pack* pack, const char* name, const void** da
         if (n == "top_children") return put(P.top_children.data(), P.top_children.size() * sizeof(GTopChild));
         if (n == "objects") return put(P.objects.data(), P.objects.size() * sizeof(GObject));
         if (n == "mesh_nodes") return put(P.nodes.data(), P.nodes.size() * sizeof(GNode));
+        if (n == "mesh_nodes4") return put(P.nodes4.data(), P.nodes4.size() * sizeof(GNode4));
         if (n == "mesh_tris") return put(P.tris.data(), P.tris.size() * sizeof(GTri));
         if (n == "meshes") return put(P.meshes.data(), P.meshes.size() * sizeof(GMesh));
         if (n == "rects") return put(P.rects.data(), P.rects.size() * sizeof(GRect));

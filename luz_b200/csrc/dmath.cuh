@@ -70,7 +70,7 @@ struct Key {
     uint32_t bounce;
 };
 
-__host__ __device__ __forceinline__ uint64_t splitmix64(uint64_t v)
+__host__ __device__ __forceinline__ constexpr uint64_t splitmix64(uint64_t v)
 {
     v += 0x9e3779b97f4a7c15ull;
     v = (v ^ (v >> 30)) * 0xbf58476d1ce4e5b9ull;
@@ -93,19 +93,60 @@ __host__ __device__ __forceinline__ uint64_t base_key(uint32_t seed, uint32_t x,
     return k;
 }
 
-__device__ __forceinline__ double dim_step(uint32_t dim, uint32_t comp)
+// Place of a dimension among the progressive ones (rank-1 lattice), -1 for the hashed ones.
+__host__ __device__ constexpr int progressive_place(uint32_t dim)
 {
-    const uint64_t key = ((uint64_t)dim + 1ull) * 0x9e3779b97f4a7c15ull ^ ((uint64_t)comp + 1ull) * 0xda942042e4dd58b5ull;
-    double s = unit24(key);
-    if (s < 0.05 || s > 0.95) s = fract(s + 0.6180339887498948);
+    switch (dim % 32u) {
+    case DIM_CAMERA: return 0;
+    case DIM_LENS: return 1;
+    case DIM_LIGHT_SURFACE_SELECTION: return 2;
+    case DIM_LIGHT_SURFACE_POINT: return 3;
+    case DIM_ENVIRONMENT_SELECTION: return 4;
+    case DIM_ENVIRONMENT_POINT: return 5;
+    case DIM_LIGHT_EMISSION_DIRECTION: return 6;
+    default: return -1;
+    }
+}
+constexpr int kProgressiveDims = 7;
+constexpr int kStepBounces = 256;   // bounces the step table covers (every render's: kMaxBounceSlots)
+
+// Lattice step of the dimension key dk = dim + bounce * 32 and the component: a function of
+// those two alone.
+__host__ __device__ constexpr double dim_step_of(uint32_t dk, uint32_t comp)
+{
+    const uint64_t key = ((uint64_t)dk + 1ull) * 0x9e3779b97f4a7c15ull ^ ((uint64_t)comp + 1ull) * 0xda942042e4dd58b5ull;
+    double s = (double)((uint32_t)(splitmix64(key) >> 32) >> 8) * (1.0 / 16777216.0);
+    if (s < 0.05 || s > 0.95) {   // fract of a value in [0, 2)
+        s = s + 0.6180339887498948;
+        if (s >= 1.0) s -= 1.0;
+    }
     return s;
 }
-__device__ __forceinline__ bool progressive(uint32_t dim)
+struct StepTable {
+    double step[kStepBounces][kProgressiveDims][2];
+};
+constexpr StepTable make_step_table()
 {
-    const uint32_t b = dim % 32u;
-    return b == DIM_CAMERA || b == DIM_LENS || b == DIM_LIGHT_SURFACE_SELECTION || b == DIM_LIGHT_SURFACE_POINT
-           || b == DIM_ENVIRONMENT_SELECTION || b == DIM_ENVIRONMENT_POINT || b == DIM_LIGHT_EMISSION_DIRECTION;
+    StepTable t{};
+    for (uint32_t b = 0; b < kStepBounces; b++)
+        for (uint32_t dim = 0; dim < 32; dim++) {
+            const int place = progressive_place(dim);
+            if (place < 0) continue;
+            for (uint32_t c = 0; c < 2; c++) t.step[b][place][c] = dim_step_of(dim + b * 32u, c);
+        }
+    return t;
 }
+// The steps of every render's bounces (28 KB). A bounce's lanes read one address, which the
+// constant cache broadcasts, where each used to hash its key again: a 64-bit splitmix and a
+// conversion per component and sample.
+static __constant__ StepTable c_steps = make_step_table();
+
+// (Every key that draws a progressive dimension has a path's or a photon's bounce, below 256.)
+__device__ __forceinline__ double dim_step(uint32_t dim, uint32_t bounce, uint32_t comp)
+{
+    return c_steps.step[bounce & (uint32_t)(kStepBounces - 1)][progressive_place(dim)][comp];
+}
+__device__ __forceinline__ bool progressive(uint32_t dim) { return progressive_place(dim) >= 0; }
 __device__ __forceinline__ uint64_t ctx_key(const Key& k, uint32_t dk)
 {
     return k.base ^ (((uint64_t)dk + 1ull) * 0x9e3779b97f4a7c15ull);
@@ -122,7 +163,7 @@ static __device__ LUZ_SAMPLER_ATTR double sample1d(const Key& k, uint32_t dim)
     const uint32_t dk = dim + k.bounce * 32u;
     if (!progressive(dim)) return hashed(k, dk, 0);
     const double shift = unit24(ctx_key(k, dk));
-    const double step = dim_step(dk, 0);
+    const double step = dim_step(dim, k.bounce, 0);
     // fract(0.5 + (s + 1) * step + shift), each operation rounded on its own as the reference computes it
     return fract(__dadd_rn(__dadd_rn(0.5, __dmul_rn((double)k.sample + 1.0, step)), shift));
 }
@@ -137,8 +178,8 @@ static __device__ LUZ_SAMPLER_ATTR S2 sample2d(const Key& k, uint32_t dim)
     const double sx = unit24(key);
     const double sy = unit24(key ^ 0xda942042e4dd58b5ull);
     const double s = (double)k.sample + 1.0;
-    return S2{(float)fract(__dadd_rn(__dadd_rn(0.5, __dmul_rn(s, dim_step(dk, 0))), sx)),
-              (float)fract(__dadd_rn(__dadd_rn(0.5, __dmul_rn(s, dim_step(dk, 1))), sy))};
+    return S2{(float)fract(__dadd_rn(__dadd_rn(0.5, __dmul_rn(s, dim_step(dim, k.bounce, 0))), sx)),
+              (float)fract(__dadd_rn(__dadd_rn(0.5, __dmul_rn(s, dim_step(dim, k.bounce, 1))), sy))};
 }
 
 constexpr float kTwoPiF = 6.28318530717958647692f;   // static_cast<float>(2.0 * D_PI)

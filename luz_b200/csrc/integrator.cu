@@ -30,6 +30,7 @@
 #include "luz_gpu.h"
 #include "nfor.h"
 #include "pack.h"
+#include "walk.cuh"
 #include "wavefront.cuh"
 
 namespace luz {
@@ -56,25 +57,17 @@ __global__ void __launch_bounds__(kBlock) k_raygen(WaveArgs w, PathBuf P, Ctrl* 
     P.queue0[p] = (uint32_t)p;
 }
 
-// ---------------------------------------------------------------------------- extend (closest hit)
+// ---------------------------------------------------------------------------- trace (closest and any hits)
 
-// Resident blocks per SM the register allocator is asked to allow, measured on
-// B200 (1080p glossy frame at 16 spp, extend / shadow stage): extend 7 blocks (72
-// registers) 35.8-35.9 ms, 8 (64) 36.8 ms, 6 (80) 37.1 ms, 5 (96, almost no spills)
-// 38.0 ms (on an earlier build with more local-memory traffic 5 blocks had led 6 and
-// 7); shadow 8 blocks 16.0 ms, 10 16.7 ms, 12 18.4 ms (shade: shade_kernels.cu).
-#ifndef LUZ_EXTEND_MIN_BLOCKS
-#define LUZ_EXTEND_MIN_BLOCKS 7
+// Resident blocks per SM the register allocator is asked to allow.
+#ifndef LUZ_TRACE_MIN_BLOCKS
+#define LUZ_TRACE_MIN_BLOCKS 8
 #endif
-#ifndef LUZ_SHADOW_MIN_BLOCKS
-#define LUZ_SHADOW_MIN_BLOCKS 8
+#ifndef LUZ_TRACE_MIN_BLOCKS_INST
+#define LUZ_TRACE_MIN_BLOCKS_INST 6
 #endif
-// The instantiations for scenes with instances (instance transform, two nested walks),
-// measured at 4-6 blocks (5 again on the final build: 85.5 against 72.0 ms):
-// 4 blocks (128 registers, a few hundred bytes of spills instead of 1-2 KB at 96) took
-// the 1e5-instance frame's extend stage from 85.1 to 71.8 ms at 4 spp (6 blocks: 85.8).
-#ifndef LUZ_EXTEND_MIN_BLOCKS_INST
-#define LUZ_EXTEND_MIN_BLOCKS_INST 4
+#ifndef LUZ_TRACE_MIN_BLOCKS_BATCH
+#define LUZ_TRACE_MIN_BLOCKS_BATCH 6
 #endif
 
 // Radiance-cache training steps: on the warm-up wave (the first sample of every pixel,
@@ -103,103 +96,158 @@ __device__ __forceinline__ void bin_append(uint32_t* bin_count, const PathBuf& P
     P.bins[cls * P.bin_stride + base + (uint32_t)__popc(peers & ((1u << lane) - 1u))] = p;
 }
 
-// Extend and shadow are instantiated per scene feature set (TF_* bits:
-// instances, volumes); a scene without them runs traversal code without the
-// instance transform or the volume sampler, and skips the per-ray sampler key.
-// COUNT instantiations add the record counts of LUZ_RENDER_COUNT; the others
-// carry no counting code (the shadow kernel counts under a runtime branch).
-template <uint32_t F, bool COUNT>
-__global__ void __launch_bounds__(kBlock, (F & TF_INSTANCE) ? LUZ_EXTEND_MIN_BLOCKS_INST : LUZ_EXTEND_MIN_BLOCKS)
-    k_extend(DScene S, WaveArgs w, PathBuf P, Ctrl* C, int bounce)
+// The volume sample of a path's rays at a bounce (VolSample's rule: drawn once, on first use).
+struct PathVolume {
+    const WaveArgs& w;
+    const PathBuf& P;
+    uint32_t p;
+    int bounce;
+    double u = 0.0;
+    bool have = false;
+    __device__ __forceinline__ PathVolume(const WaveArgs& w_, const PathBuf& P_, uint32_t p_, int b_)
+        : w(w_), P(P_), p(p_), bounce(b_)
+    {
+    }
+    __device__ __forceinline__ double get()
+    {
+        if (!have) {
+            const uint32_t pix = P.pixel[p];
+            u = sample1d(path_key(w, pix % (uint32_t)w.width, pix / (uint32_t)w.width, P.sample[p], (uint32_t)bounce),
+                         DIM_VOLUME_DISTANCE);
+            have = true;
+        }
+        return u;
+    }
+};
+
+// Rays a warp fetches at a time: 32, or fewer when the queue does not fill the grid's
+// warps, so that the rays of a short queue spread over the chip instead of sharing warps
+// (a launch lasts as long as its slowest warp, and a warp as long as the steps of all its
+// divergent rays).
+__device__ __forceinline__ uint32_t rays_per_fetch(uint32_t count)
 {
-    if constexpr ((F & TF_STAGED) != 0) stage_top_nodes(S);
-    LocalStack<true> st;
-    const uint32_t count = C->count[bounce];
+    const uint32_t warps = gridDim.x * (kBlock / 32);
+    return min(32u, max(1u, (count + warps - 1u) / warps));
+}
+__device__ __forceinline__ uint32_t fetch_rays(uint32_t* counter, uint32_t n)
+{
+    uint32_t base = 0;
+    if (lane_id() == 0) base = atomicAdd(counter, n);
+    return __shfl_sync(0xffffffffu, base, 0);
+}
+
+// Closest hits of the extension rays of `bounce`; appends each path to its shade class.
+template <uint32_t F, bool COUNT>
+__device__ __forceinline__ void trace_extension(const DScene& S, const WaveArgs& w, const PathBuf& P, Ctrl* C, int bounce,
+                                                uint2* st, WorldRays* wr)
+{
+    Walk<F, false, COUNT, PathVolume> walk;
+    walk.st = st;
+    const uint32_t count = C->count[bounce], per = rays_per_fetch(count);
     const uint32_t* q = (w.sorted_queue && bounce >= 1) ? w.sorted_queue : ((bounce & 1) ? P.queue1 : P.queue0);
     while (true) {
-        uint32_t base = 0;
-        if (lane_id() == 0) base = atomicAdd(&C->fetch_ext[bounce], 32u);
-        base = __shfl_sync(0xffffffffu, base, 0);
+        const uint32_t base = fetch_rays(&C->fetch_ext[bounce], per);
         if (base >= count) break;
-        const uint32_t i = base + lane_id();
-        const unsigned vmask = __ballot_sync(0xffffffffu, i < count);
-        if (i >= count) continue;
-        const uint32_t p = q[i];
-        const float4 o = P.ray_o[p], d = P.ray_d[p];
-        const TRay r = make_ray_x(F3{o.x, o.y, o.z}, F3{d.x, d.y, d.z}, __float_as_int(o.w), __float_as_int(d.w));
-        Key k{};
-        if constexpr ((F & TF_VOLUME) != 0) {
-            const uint32_t pix = P.pixel[p];
-            k = path_key(w, pix % (uint32_t)w.width, pix / (uint32_t)w.width, P.sample[p], (uint32_t)bounce);
+        const bool valid = lane_id() < per && base + lane_id() < count;
+        const uint32_t p = valid ? q[base + lane_id()] : 0u;
+        walk.state = WS_DONE;
+        if (valid) {
+            const float4 o = P.ray_o[p], d = P.ray_d[p];
+            walk.start(S, make_ray_x(F3{o.x, o.y, o.z}, F3{d.x, d.y, d.z}, __float_as_int(o.w), __float_as_int(d.w)),
+                       kTMin, kInf);
         }
-        VolSample vs{&k, 0.0, false};
-        const THit h = closest_hit<F>(S, r, kTMin, kInf, vs, st);
-        P.hit[p] = make_float4(h.t, h.u, h.v, __int_as_float(h.obj));
-        P.hit_prim[p] = h.prim;
-        if (P.bins) bin_append(C->bin[bounce], P, vmask, h.obj < 0 ? 0u : (uint32_t)S.obj_class[h.obj], p);
-        if constexpr (COUNT) {
-            atomicAdd(&S.counters[0], (unsigned long long)vs.nodes);
-            atomicAdd(&S.counters[1], (unsigned long long)vs.tris);
-            atomicAdd(&S.counters[2], (unsigned long long)vs.top);
-            atomicAdd(&S.counters[6], (unsigned long long)vs.bnodes);
+        PathVolume vs(w, P, p, bounce);
+        walk_warp<false>(S, walk, wr, vs);
+        const unsigned vmask = __ballot_sync(0xffffffffu, valid);
+        if (valid) {
+            const THit h = walk.h;
+            P.hit[p] = make_float4(h.t, h.u, h.v, __int_as_float(h.obj));
+            P.hit_prim[p] = h.prim;
+            if (P.bins) bin_append(C->bin[bounce], P, vmask, h.obj < 0 ? 0u : (uint32_t)S.obj_class[h.obj], p);
+            if constexpr (COUNT) {
+                atomicAdd(&S.counters[0], (unsigned long long)walk.n_nodes);
+                atomicAdd(&S.counters[1], (unsigned long long)walk.n_tris);
+                atomicAdd(&S.counters[2], (unsigned long long)walk.n_top);
+                atomicAdd(&S.counters[6], (unsigned long long)walk.n_bnodes);
+            }
         }
+        __syncwarp();
     }
 }
 
-// ---------------------------------------------------------------------------- shadow (any hit)
+// Any hits of the shadow rays emitted at `bounce`: an occluded ray clears its path's pending slot.
+template <uint32_t F, bool COUNT>
+__device__ __forceinline__ void trace_shadow(const DScene& S, const WaveArgs& w, const PathBuf& P, Ctrl* C, int bounce,
+                                             uint2* st, WorldRays* wr)
+{
+    Walk<F, true, COUNT, PathVolume> walk;
+    walk.st = st;
+    const uint32_t count = C->shadow[bounce], per = rays_per_fetch(count);
+    while (true) {
+        const uint32_t base = fetch_rays(&C->fetch_sh[bounce], per);
+        if (base >= count) break;
+        const uint32_t i = base + lane_id();
+        const bool valid = lane_id() < per && i < count;
+        walk.state = WS_DONE;
+        uint32_t tag = 0;
+        if (valid) {
+            const float4 o = P.sh_o[i], d = P.sh_d[i];
+            tag = __float_as_uint(d.w);
+            const int2 x = P.sh_x[i];
+            walk.start(S, make_ray_x(F3{o.x, o.y, o.z}, F3{d.x, d.y, d.z}, x.x, x.y), kTMin, o.w);
+        }
+        const uint32_t p = tag & 0x7fffffffu;
+        PathVolume vs(w, P, p, bounce);
+        walk_warp<false>(S, walk, wr, vs);
+        if (valid) {
+            if (walk.h.obj >= 0) {
+                if (tag & 0x80000000u) P.pend1[p] = make_float4(0.f, 0.f, 0.f, 0.f);
+                else P.pend0[p] = make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+            if constexpr (COUNT) {
+                atomicAdd(&S.counters[3], (unsigned long long)walk.n_nodes);
+                atomicAdd(&S.counters[4], (unsigned long long)walk.n_tris);
+                atomicAdd(&S.counters[5], (unsigned long long)walk.n_top);
+                atomicAdd(&S.counters[7], (unsigned long long)walk.n_bnodes);
+            }
+        }
+        __syncwarp();
+    }
+}
 
-// (The record counts stay a runtime branch here: an instantiation without them
-// measured 2.6x slower on B200, at 2.3 instead of 7.0 active threads per warp
-// instruction for the same rays, a reconvergence effect of the smaller loop body.)
-template <uint32_t F>
-__global__ void __launch_bounds__(kBlock, LUZ_SHADOW_MIN_BLOCKS) k_shadow(DScene S, WaveArgs w, PathBuf P, Ctrl* C, int bounce)
+// The trace stage before the shading of `bounce`: the extension rays of `bounce` and the
+// shadow rays that bounce - 1 emitted, in one launch (what: TRACE_EXTEND | TRACE_SHADOW).
+// The two are independent, both must end before the bounce is shaded, and a launch of
+// either alone lasts as long as its slowest rays: together one's last rays run beside the
+// other's first. Instantiated per scene feature set (TF_* bits: instances, volumes; a scene
+// without them runs traversal code without the instance transform or the volume sampler);
+// COUNT instantiations add the record counts of LUZ_RENDER_COUNT.
+enum TraceWhat : int { TRACE_EXTEND = 1, TRACE_SHADOW = 2 };
+
+template <uint32_t F, bool COUNT>
+__global__ void __launch_bounds__(kBlock, (F & TF_INSTANCE) ? LUZ_TRACE_MIN_BLOCKS_INST : LUZ_TRACE_MIN_BLOCKS)
+    k_trace(DScene S, WaveArgs w, PathBuf P, Ctrl* C, int bounce, int what)
 {
     if constexpr ((F & TF_STAGED) != 0) stage_top_nodes(S);
-    LocalStack<false> st;
-    const uint32_t count = C->shadow[bounce];
-    while (true) {
-        uint32_t base = 0;
-        if (lane_id() == 0) base = atomicAdd(&C->fetch_sh[bounce], 32u);
-        base = __shfl_sync(0xffffffffu, base, 0);
-        if (base >= count) break;
-        const uint32_t i = base + lane_id();
-        if (i >= count) continue;
-        const float4 o = P.sh_o[i], d = P.sh_d[i];
-        const uint32_t tag = __float_as_uint(d.w);
-        const uint32_t p = tag & 0x7fffffffu;
-        const int2 x = P.sh_x[i];
-        const TRay r = make_ray_x(F3{o.x, o.y, o.z}, F3{d.x, d.y, d.z}, x.x, x.y);
-        Key k{};
-        if constexpr ((F & TF_VOLUME) != 0) {
-            const uint32_t pix = P.pixel[p];
-            k = path_key(w, pix % (uint32_t)w.width, pix / (uint32_t)w.width, P.sample[p], (uint32_t)bounce);
-        }
-        VolSample vs{&k, 0.0, false};
-        if (any_hit<F>(S, r, kTMin, o.w, vs, st)) {
-            if (tag & 0x80000000u) P.pend1[p] = make_float4(0.f, 0.f, 0.f, 0.f);
-            else P.pend0[p] = make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-        if (S.counters) {
-            atomicAdd(&S.counters[3], (unsigned long long)vs.nodes);
-            atomicAdd(&S.counters[4], (unsigned long long)vs.tris);
-            atomicAdd(&S.counters[5], (unsigned long long)vs.top);
-            atomicAdd(&S.counters[7], (unsigned long long)vs.bnodes);
-        }
+    WorldRays* wr = nullptr;
+    if constexpr ((F & TF_INSTANCE) != 0) {
+        __shared__ WorldRays s_world;
+        wr = &s_world;
     }
+    uint2 st[kWalkStack];
+    if (what & TRACE_EXTEND) trace_extension<F, COUNT>(S, w, P, C, bounce, st, wr);
+    if (what & TRACE_SHADOW) trace_shadow<F, COUNT>(S, w, P, C, bounce - 1, st, wr);
 }
 
-using TraceKernel = void (*)(DScene, WaveArgs, PathBuf, Ctrl*, int);
+using TraceKernel = void (*)(DScene, WaveArgs, PathBuf, Ctrl*, int, int);
 // Indexed [count][features | staged]: TF_STAGED variants read the scene's top
 // collapsed nodes from shared memory (a tuning choice, off by default: on the
 // 1080p glossy frame they measured 2.5% slower, the nodes being L1-resident).
-const TraceKernel kExtendKernels[2][8] = {
-    {k_extend<0, false>, k_extend<1, false>, k_extend<2, false>, k_extend<3, false>,
-     k_extend<4, false>, k_extend<5, false>, k_extend<6, false>, k_extend<7, false>},
-    {k_extend<0, true>, k_extend<1, true>, k_extend<2, true>, k_extend<3, true>,
-     k_extend<4, true>, k_extend<5, true>, k_extend<6, true>, k_extend<7, true>}};
-const TraceKernel kShadowKernels[8] = {k_shadow<0>, k_shadow<1>, k_shadow<2>, k_shadow<3>,
-                                       k_shadow<4>, k_shadow<5>, k_shadow<6>, k_shadow<7>};
-
+const TraceKernel kTraceKernels[2][8] = {
+    {k_trace<0, false>, k_trace<1, false>, k_trace<2, false>, k_trace<3, false>,
+     k_trace<4, false>, k_trace<5, false>, k_trace<6, false>, k_trace<7, false>},
+    {k_trace<0, true>, k_trace<1, true>, k_trace<2, true>, k_trace<3, true>,
+     k_trace<4, true>, k_trace<5, true>, k_trace<6, true>, k_trace<7, true>}};
 
 // ---------------------------------------------------------------------------- coherence sort
 //
@@ -343,69 +391,88 @@ __device__ __forceinline__ void count_by_scene(unsigned mask, uint32_t sid, unsi
     if ((int)lane_id() == __ffs(peers) - 1) atomicAdd(&counts[sid], (unsigned long long)__popc(peers));
 }
 
-__global__ void __launch_bounds__(kBlock, LUZ_EXTEND_MIN_BLOCKS) k_extend_batch(const DScene* __restrict__ scenes,
-                                                                               const WaveArgs* __restrict__ segs,
-                                                                               PathBuf P, Ctrl* C, int bounce,
-                                                                               unsigned long long* ext_rays)
+__device__ __forceinline__ void trace_extension_batch(const DScene* __restrict__ scenes, const WaveArgs* __restrict__ segs,
+                                                      const PathBuf& P, Ctrl* C, int bounce, unsigned long long* ext_rays,
+                                                      uint2* st, WorldRays* wr)
 {
-    LocalStack<true> st;
-    const uint32_t count = C->count[bounce];
+    Walk<TF_ALL, false, false, PathVolume> walk;
+    walk.st = st;
+    const uint32_t count = C->count[bounce], per = rays_per_fetch(count);
     const uint32_t* q = (bounce & 1) ? P.queue1 : P.queue0;
     while (true) {
-        uint32_t base = 0;
-        if (lane_id() == 0) base = atomicAdd(&C->fetch_ext[bounce], 32u);
-        base = __shfl_sync(0xffffffffu, base, 0);
+        const uint32_t base = fetch_rays(&C->fetch_ext[bounce], per);
         if (base >= count) break;
-        const uint32_t i = base + lane_id();
-        const unsigned vmask = __ballot_sync(0xffffffffu, i < count);
-        if (i >= count) continue;
-        const uint32_t p = q[i];
+        const bool valid = lane_id() < per && base + lane_id() < count;
+        const uint32_t p = q[valid ? base + lane_id() : base];
         const WaveArgs& w = segs[P.seg[p]];
         const DScene& S = scenes[w.batch_scene];
-        const float4 o = P.ray_o[p], d = P.ray_d[p];
-        const TRay r = make_ray_x(F3{o.x, o.y, o.z}, F3{d.x, d.y, d.z}, __float_as_int(o.w), __float_as_int(d.w));
-        const uint32_t pix = P.pixel[p];
-        Key k = path_key(w, pix % (uint32_t)w.width, pix / (uint32_t)w.width, P.sample[p], (uint32_t)bounce);
-        VolSample vs{&k, 0.0, false};
-        const THit h = closest_hit<TF_ALL>(S, r, kTMin, kInf, vs, st);
-        P.hit[p] = make_float4(h.t, h.u, h.v, __int_as_float(h.obj));
-        P.hit_prim[p] = h.prim;
-        bin_append(C->bin[bounce], P, vmask, h.obj < 0 ? 0u : (uint32_t)S.obj_class[h.obj], p);
-        count_by_scene(vmask, (uint32_t)w.batch_scene, ext_rays);
+        walk.state = WS_DONE;
+        if (valid) {
+            const float4 o = P.ray_o[p], d = P.ray_d[p];
+            walk.start(S, make_ray_x(F3{o.x, o.y, o.z}, F3{d.x, d.y, d.z}, __float_as_int(o.w), __float_as_int(d.w)),
+                       kTMin, kInf);
+        }
+        PathVolume vs(w, P, p, bounce);
+        walk_warp<true>(S, walk, wr, vs);
+        const unsigned vmask = __ballot_sync(0xffffffffu, valid);
+        if (valid) {
+            const THit h = walk.h;
+            P.hit[p] = make_float4(h.t, h.u, h.v, __int_as_float(h.obj));
+            P.hit_prim[p] = h.prim;
+            bin_append(C->bin[bounce], P, vmask, h.obj < 0 ? 0u : (uint32_t)S.obj_class[h.obj], p);
+            count_by_scene(vmask, (uint32_t)w.batch_scene, ext_rays);
+        }
+        __syncwarp();
     }
 }
 
-__global__ void __launch_bounds__(kBlock, LUZ_SHADOW_MIN_BLOCKS) k_shadow_batch(const DScene* __restrict__ scenes,
-                                                                               const WaveArgs* __restrict__ segs,
-                                                                               PathBuf P, Ctrl* C, int bounce,
-                                                                               unsigned long long* sh_rays)
+__device__ __forceinline__ void trace_shadow_batch(const DScene* __restrict__ scenes, const WaveArgs* __restrict__ segs,
+                                                   const PathBuf& P, Ctrl* C, int bounce, unsigned long long* sh_rays,
+                                                   uint2* st, WorldRays* wr)
 {
-    LocalStack<false> st;
-    const uint32_t count = C->shadow[bounce];
+    Walk<TF_ALL, true, false, PathVolume> walk;
+    walk.st = st;
+    const uint32_t count = C->shadow[bounce], per = rays_per_fetch(count);
     while (true) {
-        uint32_t base = 0;
-        if (lane_id() == 0) base = atomicAdd(&C->fetch_sh[bounce], 32u);
-        base = __shfl_sync(0xffffffffu, base, 0);
+        const uint32_t base = fetch_rays(&C->fetch_sh[bounce], per);
         if (base >= count) break;
-        const uint32_t i = base + lane_id();
-        const unsigned vmask = __ballot_sync(0xffffffffu, i < count);
-        if (i >= count) continue;
-        const float4 o = P.sh_o[i], d = P.sh_d[i];
-        const uint32_t tag = __float_as_uint(d.w);
+        const bool valid = lane_id() < per && base + lane_id() < count;
+        const uint32_t i = valid ? base + lane_id() : base;
+        const uint32_t tag = __float_as_uint(P.sh_d[i].w);
         const uint32_t p = tag & 0x7fffffffu;
         const WaveArgs& w = segs[P.seg[p]];
         const DScene& S = scenes[w.batch_scene];
-        const int2 x = P.sh_x[i];
-        const TRay r = make_ray_x(F3{o.x, o.y, o.z}, F3{d.x, d.y, d.z}, x.x, x.y);
-        const uint32_t pix = P.pixel[p];
-        Key k = path_key(w, pix % (uint32_t)w.width, pix / (uint32_t)w.width, P.sample[p], (uint32_t)bounce);
-        VolSample vs{&k, 0.0, false};
-        if (any_hit<TF_ALL>(S, r, kTMin, o.w, vs, st)) {
-            if (tag & 0x80000000u) P.pend1[p] = make_float4(0.f, 0.f, 0.f, 0.f);
-            else P.pend0[p] = make_float4(0.f, 0.f, 0.f, 0.f);
+        walk.state = WS_DONE;
+        if (valid) {
+            const float4 o = P.sh_o[i], d = P.sh_d[i];
+            const int2 x = P.sh_x[i];
+            walk.start(S, make_ray_x(F3{o.x, o.y, o.z}, F3{d.x, d.y, d.z}, x.x, x.y), kTMin, o.w);
         }
-        count_by_scene(vmask, (uint32_t)w.batch_scene, sh_rays);
+        PathVolume vs(w, P, p, bounce);
+        walk_warp<true>(S, walk, wr, vs);
+        const unsigned vmask = __ballot_sync(0xffffffffu, valid);
+        if (valid) {
+            if (walk.h.obj >= 0) {
+                if (tag & 0x80000000u) P.pend1[p] = make_float4(0.f, 0.f, 0.f, 0.f);
+                else P.pend0[p] = make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+            count_by_scene(vmask, (uint32_t)w.batch_scene, sh_rays);
+        }
+        __syncwarp();
     }
+}
+
+// k_trace over the rays of many scenes.
+__global__ void __launch_bounds__(kBlock, LUZ_TRACE_MIN_BLOCKS_BATCH) k_trace_batch(const DScene* __restrict__ scenes,
+                                                                                   const WaveArgs* __restrict__ segs,
+                                                                                   PathBuf P, Ctrl* C, int bounce, int what,
+                                                                                   unsigned long long* ext_rays,
+                                                                                   unsigned long long* sh_rays)
+{
+    __shared__ WorldRays s_world;
+    uint2 st[kWalkStack];
+    if (what & TRACE_EXTEND) trace_extension_batch(scenes, segs, P, C, bounce, ext_rays, st, &s_world);
+    if (what & TRACE_SHADOW) trace_shadow_batch(scenes, segs, P, C, bounce - 1, sh_rays, st, &s_world);
 }
 
 // k_accumulate over the segments of a multi-scene wave (blockIdx.y = segment): each
@@ -710,36 +777,49 @@ __global__ void k_converge(AdaptiveRule R, uint32_t used, const uint32_t* act, u
 
 // ---------------------------------------------------------------------------- ray batches
 
-// luz_gpu_trace_rays: one ray per thread through the traversal instantiation
-// the extend / shadow kernels use for this scene.
-template <uint32_t F>
-__global__ void k_trace_rays(DScene S, const float* rays, int64_t n, int any, uint32_t seed, const int32_t* vkey,
-                             LuzHit* out)
+// luz_gpu_trace_rays: one ray per lane through the walk the extend / shadow kernels
+// use for this scene.
+template <uint32_t F, bool ANY>
+__device__ __forceinline__ THit trace_ray(const DScene& S, const float* r, bool valid, WorldRays* wr, VolSample& vs)
 {
+    uint2 st[kWalkStack];
+    Walk<F, ANY, false, VolSample> walk;
+    walk.st = st;
+    walk.state = WS_DONE;
+    if (valid) walk.start(S, make_ray(F3{r[0], r[1], r[2]}, F3{r[4], r[5], r[6]}), r[3], r[7]);
+    walk_warp<false>(S, walk, wr, vs);
+    return walk.h;
+}
+
+template <uint32_t F>
+__global__ void __launch_bounds__(kWalkBlock) k_trace_rays(DScene S, const float* rays, int64_t n, int any, uint32_t seed,
+                                                           const int32_t* vkey, LuzHit* out)
+{
+    WorldRays* wr = nullptr;
+    if constexpr ((F & TF_INSTANCE) != 0) {
+        __shared__ WorldRays s_world;
+        wr = &s_world;
+    }
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float* r = rays + 8 * i;
-    const TRay ray = make_ray(F3{r[0], r[1], r[2]}, F3{r[4], r[5], r[6]});
+    const bool valid = i < n;
+    const float* r = rays + 8 * (valid ? i : 0);
     Key k;
-    if (vkey) k = Key{base_key(seed, (uint32_t)vkey[4 * i], (uint32_t)vkey[4 * i + 1], 0), (uint32_t)vkey[4 * i + 2],
-                      (uint32_t)vkey[4 * i + 3]};
+    if (vkey && valid) k = Key{base_key(seed, (uint32_t)vkey[4 * i], (uint32_t)vkey[4 * i + 1], 0),
+                               (uint32_t)vkey[4 * i + 2], (uint32_t)vkey[4 * i + 3]};
     else k = Key{base_key(seed, 0, 0, 0), 0, 0};
     VolSample vs{&k, 0.0, false};
+    const THit h = any ? trace_ray<F, true>(S, r, valid, wr, vs) : trace_ray<F, false>(S, r, valid, wr, vs);
+    if (!valid) return;
     LuzHit o;
-    LocalStack<true> st;
     if (any) {
-        const bool occ = any_hit<F>(S, ray, r[3], r[7], vs, st);
-        o = LuzHit{0.f, occ ? 0 : -1, 0, 0.f, 0.f};
+        o = LuzHit{0.f, h.obj >= 0 ? 0 : -1, 0, 0.f, 0.f};
+    } else if (h.obj < 0) {
+        o = LuzHit{kInf, -1, -1, 0.f, 0.f};
     } else {
-        const THit h = closest_hit<F>(S, ray, r[3], r[7], vs, st);
-        if (h.obj < 0) {
-            o = LuzHit{kInf, -1, -1, 0.f, 0.f};
-        } else {
-            const GObject O = S.objects[h.obj];
-            int32_t prim = h.prim;
-            if (O.kind == OK_MESH || O.kind == OK_INSTANCE) prim = (int32_t)load_tri(S.tris, (uint32_t)h.prim).orig;
-            o = LuzHit{h.t, O.id, prim, h.u, h.v};
-        }
+        const GObject O = S.objects[h.obj];
+        int32_t prim = h.prim;
+        if (O.kind == OK_MESH || O.kind == OK_INSTANCE) prim = (int32_t)load_tri(S.tris, (uint32_t)h.prim).orig;
+        o = LuzHit{h.t, O.id, prim, h.u, h.v};
     }
     out[i] = o;
 }
@@ -779,7 +859,7 @@ __global__ void __launch_bounds__(128) k_photons(DScene S, uint32_t seed, int ma
     if (!valid_positive(thr)) return;
     TRay ray = make_ray(e.pos + e.dir * (2.0f * kTMin), e.dir);
     bool caustic = false;
-    LocalStack<true> st;
+    LocalStack st;
     for (int b = 0; b <= max_bounces; b++) {
         k.bounce = (uint32_t)b;
         VolSample vs{&k, 0.0, false};
@@ -948,14 +1028,13 @@ struct luz_gpu_scene {
     float* out_dev = nullptr;        // luz_gpu_render: device film of per-pixel means
     int64_t out_cap = 0;
     int sms = 0;
-    int occ_ext = 1, occ_shade = 1, occ_sh = 1;
+    int occ_trace = 1, occ_shade = 1;
     LuzTuneParams tune{};            // luz_gpu_scene_set_tuning / luz_gpu_autotune; zeros = defaults
     // multi-scene batches copy the scene arrays into their geometry arena: byte offset of
     // each array pointer inside DScene and the array's size; uid / version name the
     // content (version changes with texels or the caustic map)
     std::vector<std::pair<std::size_t, std::size_t>> arena_fields;
     uint64_t uid = 0, version = 0;
-    TraceKernel extend = nullptr, shadow = nullptr;   // instantiations for this scene's features
     ShadeKernel shade = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     // caustic photon map: buffers grown on demand; the map is kept while the
@@ -1184,19 +1263,24 @@ void launch_bounces(luz_gpu_scene* s, const WaveArgs& w, cudaStream_t st, int64_
                     ShadeKernel shade, const PathBuf& pb, Ctrl* ctrl)
 {
     auto blocks = [](int tuned, int occ) { return tuned > 0 ? std::min(tuned, occ) : occ; };
-    const int g_ext = s->sms * blocks(s->tune.extend_blocks_per_sm, s->occ_ext);
-    const int g_sh = s->sms * blocks(s->tune.shadow_blocks_per_sm, s->occ_sh);
-    const int g_shade = s->sms * blocks(s->tune.shade_blocks_per_sm, s->occ_shade);
+    // no more blocks than the wave's rays could keep busy
+    const int64_t need = std::max<int64_t>(1, (w.n + kBlock - 1) / kBlock);
+    auto grid = [&](int per_sm, int64_t rays) {
+        return (unsigned)std::min<int64_t>((int64_t)s->sms * per_sm, rays * need);
+    };
+    const unsigned g_ext = grid(blocks(s->tune.extend_blocks_per_sm, s->occ_trace), 32);
+    const unsigned g_sh = grid(blocks(s->tune.shadow_blocks_per_sm, s->occ_trace), 64);
+    const unsigned g_shade = grid(blocks(s->tune.shade_blocks_per_sm, s->occ_shade), 1);
     if (!shade) shade = s->shade;
     const int count = s->ds.counters ? 1 : 0;   // LUZ_RENDER_COUNT renders run the counting instantiations
     const uint32_t kv = (s->ds.k.features & TF_ALL) | (s->tune.staged_top_nodes && s->ds.top4_count ? TF_STAGED : 0u);
-    const TraceKernel extend = kExtendKernels[count][kv];
-    const TraceKernel shadow = kShadowKernels[kv];
+    const TraceKernel trace = kTraceKernels[count][kv];
     WaveArgs ws = w;
     const bool sort = s->tune.sort_rays != 0 && pb.qsort;
     if (sort) ws.sorted_queue = pb.qsort;
-    for (int b = 0; b <= w.max_bounces; b++) {
-        if (sort && b >= 1) {
+    for (int b = 0; b <= w.max_bounces + 1; b++) {
+        const bool ext = b <= w.max_bounces;
+        if (ext && sort && b >= 1) {
             const uint32_t* q = (b & 1) ? pb.queue1 : pb.queue0;
             CK(cudaMemsetAsync(pb.sort_hist, 0, sizeof(uint32_t) * kSortBins, st));
             k_sort_keys<<<s->sms * 8, 256, 0, st>>>(ctrl, b, q, pb, s->ds.k);
@@ -1204,16 +1288,27 @@ void launch_bounces(luz_gpu_scene* s, const WaveArgs& w, cudaStream_t st, int64_
             k_sort_scatter<<<s->sms * 8, 256, 0, st>>>(ctrl, b, q, pb);
             launches += 3;
         }
-        T.mark(st, 0, true);
-        extend<<<g_ext, kBlock, 0, st>>>(s->ds, ws, pb, ctrl, b);
-        T.mark(st, 0, false);
+        if (T.on) {   // stage timing: one launch per stage
+            if (b >= 1) {
+                T.mark(st, 2, true);
+                trace<<<g_sh, kBlock, 0, st>>>(s->ds, ws, pb, ctrl, b, TRACE_SHADOW);
+                T.mark(st, 2, false);
+                launches++;
+            }
+            if (!ext) break;
+            T.mark(st, 0, true);
+            trace<<<g_ext, kBlock, 0, st>>>(s->ds, ws, pb, ctrl, b, TRACE_EXTEND);
+            T.mark(st, 0, false);
+        } else {
+            trace<<<ext ? g_ext : g_sh, kBlock, 0, st>>>(s->ds, ws, pb, ctrl, b,
+                                                         (ext ? TRACE_EXTEND : 0) | (b >= 1 ? TRACE_SHADOW : 0));
+        }
+        launches++;
+        if (!ext) break;
         T.mark(st, 1, true);
-        shade<<<g_shade, kBlock, 0, st>>>(s->dds, w, pb, ctrl, b);
+        shade<<<g_shade, kShadeBlock, 0, st>>>(s->dds, w, pb, ctrl, b);
         T.mark(st, 1, false);
-        T.mark(st, 2, true);
-        shadow<<<g_sh, kBlock, 0, st>>>(s->ds, w, pb, ctrl, b);
-        T.mark(st, 2, false);
-        launches += 3;
+        launches++;
     }
     CK(cudaGetLastError());
 }
@@ -2262,11 +2357,10 @@ std::vector<std::vector<WaveArgs>> batch_waves(luz_gpu_scene* const* scenes, con
 // into a graph: every kernel reads the wave's size from device memory.
 cudaGraphExec_t batch_graph(BatchContext& C, const BatchWaveHeader* hdr, int max_b, int64_t cap_paths,
                             int64_t max_pix, int64_t max_segs, double* const* d_films, unsigned long long* d_rays,
-                            int32_t count, bool caustics, int sms, int occ_ext, int occ_sh, int occ_shade,
+                            int32_t count, bool caustics, int sms, int occ_trace, int occ_shade,
                             int64_t& launches)
 {
     (void)hdr;
-    (void)count;
     const BatchShadeKernel shade = batch_shade_kernel(caustics ? 1 : 0);
     cudaGraph_t g = nullptr;
     CK(cudaStreamBeginCapture(C.st, cudaStreamCaptureModeThreadLocal));
@@ -2274,11 +2368,14 @@ cudaGraphExec_t batch_graph(BatchContext& C, const BatchWaveHeader* hdr, int max
         CK(cudaMemsetAsync(C.ctrl, 0, sizeof(Ctrl), C.st));
         k_raygen_batch<<<(unsigned)((cap_paths + kBlock - 1) / kBlock), kBlock, 0, C.st>>>(C.d_segs, hdr, C.pb, C.ctrl);
         launches++;
-        for (int b = 0; b <= max_b; b++) {
-            k_extend_batch<<<sms * occ_ext, kBlock, 0, C.st>>>(C.d_scenes, C.d_segs, C.pb, C.ctrl, b, d_rays);
-            shade<<<sms * occ_shade, kBlock, 0, C.st>>>(C.d_scenes, C.d_segs, C.pb, C.ctrl, b);
-            k_shadow_batch<<<sms * occ_sh, kBlock, 0, C.st>>>(C.d_scenes, C.d_segs, C.pb, C.ctrl, b, d_rays + count);
-            launches += 3;
+        for (int b = 0; b <= max_b + 1; b++) {
+            k_trace_batch<<<sms * occ_trace, kBlock, 0, C.st>>>(C.d_scenes, C.d_segs, C.pb, C.ctrl, b,
+                                                               (b <= max_b ? TRACE_EXTEND : 0) | (b >= 1 ? TRACE_SHADOW : 0),
+                                                               d_rays, d_rays + count);
+            launches++;
+            if (b > max_b) break;
+            shade<<<sms * occ_shade, kShadeBlock, 0, C.st>>>(C.d_scenes, C.d_segs, C.pb, C.ctrl, b);
+            launches++;
         }
         dim3 ag((unsigned)((max_pix + 127) / 128), (unsigned)max_segs);
         k_accumulate_batch<<<ag, 128, 0, C.st>>>(C.d_segs, hdr, C.pb, d_films);
@@ -2349,12 +2446,10 @@ int batch_render(luz_gpu_scene* const* scenes, const LuzRenderParams* params, in
         CK(cudaMemcpyAsync(d_films, hf.data(), sizeof(double*) * (std::size_t)count, cudaMemcpyHostToDevice, st));
         CK(cudaStreamSynchronize(st));
     }
-    int occ_ext = 1, occ_sh = 1, occ_shade = 1;
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_ext, k_extend_batch, kBlock, 0));
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_sh, k_shadow_batch, kBlock, 0));
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_shade, batch_shade_kernel(caustics ? 1 : 0), kBlock, 0));
-    occ_ext = std::max(1, occ_ext);
-    occ_sh = std::max(1, occ_sh);
+    int occ_trace = 1, occ_shade = 1;
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_trace, k_trace_batch, kBlock, 0));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_shade, batch_shade_kernel(caustics ? 1 : 0), kShadeBlock, 0));
+    occ_trace = std::max(1, occ_trace);
     occ_shade = std::max(1, occ_shade);
     const int sms = scenes[0]->sms;
 
@@ -2386,7 +2481,7 @@ int batch_render(luz_gpu_scene* const* scenes, const LuzRenderParams* params, in
             for (const WaveArgs& w : wv) pix_max = std::max<int64_t>(pix_max, w.pix_count);
         }
         cudaGraphExec_t ex = batch_graph(C, hdr, max_b, wave_max, pix_max, segs_max, d_films, d_rays, count, caustics,
-                                         sms, occ_ext, occ_sh, occ_shade, launches);
+                                         sms, occ_trace, occ_shade, launches);
         CK(cudaMemsetAsync(films, 0, sizeof(double) * (std::size_t)film_doubles, st));
         CK(cudaMemsetAsync(d_rays, 0, sizeof(unsigned long long) * 2 * (std::size_t)count, st));
         CK(cudaEventRecord(C.ev0, st));
@@ -2590,13 +2685,7 @@ int do_render_noalloc(luz_gpu_scene* s, const LuzRenderParams* p, float* d_out, 
             w.list_mode = 0;
             CK(cudaMemsetAsync(A.ctrl, 0, sizeof(Ctrl), st));
             k_raygen<<<(unsigned)((w.n + kBlock - 1) / kBlock), kBlock, 0, st>>>(w, A.pb, A.ctrl);
-            const int g_ext = s->sms * s->occ_ext, g_sh = s->sms * s->occ_sh, g_shade = s->sms * s->occ_shade;
-            for (int b = 0; b <= w.max_bounces; b++) {
-                s->extend<<<g_ext, kBlock, 0, st>>>(s->ds, w, A.pb, A.ctrl, b);
-                s->shade<<<g_shade, kBlock, 0, st>>>(s->dds, w, A.pb, A.ctrl, b);
-                s->shadow<<<g_sh, kBlock, 0, st>>>(s->ds, w, A.pb, A.ctrl, b);
-                launches += 3;
-            }
+            launch_bounces(s, w, st, launches, T, nullptr, A.pb, A.ctrl);
             k_accumulate<<<(unsigned)((pc + 127) / 128), 128, 0, st>>>(w, A.pb, A.film);
             k_tally<<<1, 1, 0, st>>>(A.ctrl, w.max_bounces, A.totals);
             launches += 3;
@@ -2729,15 +2818,11 @@ int luz_gpu_scene_create(const LuzSceneDesc* desc, int32_t device, luz_gpu_scene
         CK(cudaGetDeviceProperties(&prop, device));
         s->sms = prop.multiProcessorCount;
         const int feat = P.consts.features & TF_ALL;
-        s->extend = kExtendKernels[0][feat];
-        s->shadow = kShadowKernels[feat];
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&s->occ_ext, s->extend, kBlock, 0));
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&s->occ_trace, kTraceKernels[0][feat], kBlock, 0));
         s->shade = shade_kernel(P.consts.caustics.enabled ? 1 : 0);
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&s->occ_shade, s->shade, kBlock, 0));
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&s->occ_sh, s->shadow, kBlock, 0));
-        s->occ_ext = std::max(1, s->occ_ext);
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&s->occ_shade, s->shade, kShadeBlock, 0));
+        s->occ_trace = std::max(1, s->occ_trace);
         s->occ_shade = std::max(1, s->occ_shade);
-        s->occ_sh = std::max(1, s->occ_sh);
         *out = s.release();
         return LUZ_OK;
     });
@@ -2864,16 +2949,16 @@ int luz_gpu_autotune(luz_gpu_scene* s, const LuzRenderParams* p, LuzTuneParams* 
                 t.wave_paths = wave;
                 consider(t);
             }
-            for (int b : {s->occ_ext - 1, s->occ_ext}) {
-                if (b < 1 || b == (best.extend_blocks_per_sm ? best.extend_blocks_per_sm : s->occ_ext)) continue;
+            for (int b : {s->occ_trace - 1, s->occ_trace}) {
+                if (b < 1 || b == (best.extend_blocks_per_sm ? best.extend_blocks_per_sm : s->occ_trace)) continue;
                 LuzTuneParams t = best;
-                t.extend_blocks_per_sm = b == s->occ_ext ? 0 : b;
+                t.extend_blocks_per_sm = b == s->occ_trace ? 0 : b;
                 consider(t);
             }
-            for (int b : {s->occ_sh / 2, s->occ_sh}) {
-                if (b < 1 || b == (best.shadow_blocks_per_sm ? best.shadow_blocks_per_sm : s->occ_sh)) continue;
+            for (int b : {s->occ_trace / 2, s->occ_trace}) {
+                if (b < 1 || b == (best.shadow_blocks_per_sm ? best.shadow_blocks_per_sm : s->occ_trace)) continue;
                 LuzTuneParams t = best;
-                t.shadow_blocks_per_sm = b == s->occ_sh ? 0 : b;
+                t.shadow_blocks_per_sm = b == s->occ_trace ? 0 : b;
                 consider(t);
             }
             s->tune = best;
@@ -3258,9 +3343,7 @@ int do_render_cached(luz_gpu_scene* s, luz_gpu_cache* c, const LuzRenderParams* 
     double* film = D.get<double>(3 * npix, st);
     float* d_out = D.get<float>(3 * npix, st);
     const ShadeKernel shade_cached = shade_kernel(2);
-    int occ = 1;
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, shade_cached, kBlock, 0));
-    occ = std::max(1, occ);
+    StageTimer T;
 
     WaveArgs w = base_args(s, p);
     const GSceneConst& K = s->pack->consts;
@@ -3278,7 +3361,6 @@ int do_render_cached(luz_gpu_scene* s, luz_gpu_cache* c, const LuzRenderParams* 
     CK(cudaMemcpyAsync(s->dds, &s->ds, sizeof(DScene), cudaMemcpyHostToDevice, st));
     CK(cudaMemsetAsync(s->totals, 0, 2 * sizeof(unsigned long long), st));
     CK(cudaEventRecord(s->ev0, st));
-    const int g_ext = s->sms * s->occ_ext, g_sh = s->sms * s->occ_sh, g_shade = s->sms * occ;
     const int batch = c->prm.batch;
     int64_t launches = 0, waves = 0;
     // The first sample of every pixel is rendered plain, every path training the
@@ -3306,11 +3388,7 @@ int do_render_cached(luz_gpu_scene* s, luz_gpu_cache* c, const LuzRenderParams* 
             CK(cudaMemsetAsync(tflag, 0, (std::size_t)w.n, st));
             CK(cudaMemsetAsync(c->loss, 0, sizeof(float), st));
             k_raygen<<<(unsigned)((w.n + kBlock - 1) / kBlock), kBlock, 0, st>>>(w, s->pb, s->ctrl);
-            for (int b = 0; b <= w.max_bounces; b++) {
-                s->extend<<<g_ext, kBlock, 0, st>>>(s->ds, w, s->pb, s->ctrl, b);
-                shade_cached<<<g_shade, kBlock, 0, st>>>(s->dds, w, s->pb, s->ctrl, b);
-                s->shadow<<<g_sh, kBlock, 0, st>>>(s->ds, w, s->pb, s->ctrl, b);
-            }
+            launch_bounces(s, w, st, launches, T, shade_cached, s->pb, s->ctrl);
             k_cache_infer<<<(unsigned)(2 * s->sms), 128, kCacheInferSmem, st>>>(q, counts, 0, c->Wf, nullptr, s->pb.rad);
             k_cache_targets<<<(unsigned)((w.n + 255) / 256), 256, 0, st>>>(w, s->pb, rows, counts + 1);
             // about n / train_every rows: one step per batch of them (at most kCacheWaveSteps);
@@ -3323,7 +3401,7 @@ int do_render_cached(luz_gpu_scene* s, luz_gpu_cache* c, const LuzRenderParams* 
             k_accumulate<<<(unsigned)((pc + 127) / 128), 128, 0, st>>>(w, s->pb, film);
             k_tally<<<1, 1, 0, st>>>(s->ctrl, w.max_bounces, s->totals);
             CK(cudaGetLastError());
-            launches += 3 * (w.max_bounces + 1) + 6 + 3 * steps;
+            launches += 6 + 3 * steps;
             waves++;
         }
         sb += sc;

@@ -83,24 +83,29 @@ struct alignas(16) GNode {
     uint32_t pad0, pad1;
 };
 
-// Collapsed mesh BVH node (160 B): a binary node N together with its two
-// children L and R. It holds the boxes of L and R and of up to four
-// grandchildren: slots 0-1 are L's children (or L itself, slot 1 empty, when L
-// is a leaf), slots 2-3 are R's. A traversal step over it visits exactly the
-// entries the binary near-first traversal would visit after N, L and R, in the
-// same order (see trace.cuh). ref: node4 index, leaf ref, or kEmptySlot.
+// Collapsed mesh BVH node (128 B, one cache line): a binary node N together with its
+// two children L and R. It holds the boxes of up to four grandchildren: slots 0-1 are
+// L's children (or L itself, slot 1 empty, when L is a leaf), slots 2-3 are R's. The
+// boxes of L and R are not stored: they are the unions of their slots' boxes. A
+// traversal step over it visits exactly the entries the binary near-first traversal
+// would visit after N, L and R, in the same order (see trace.cuh). Plane coordinates
+// are grouped by axis, so that the four planes a ray meets first along an axis are one
+// 16-byte load at an address that the ray's sign on that axis selects (lo and hi lie 64
+// bytes apart). An empty slot's box is inverted (lo = kEmptyPlane, hi = -kEmptyPlane):
+// no ray meets it. ref: node4 index, leaf ref, or kEmptySlot.
+constexpr float kEmptyPlane = 3.0e38f;
 constexpr uint32_t kEmptySlot = 0xffffffffu;
 // Collapsed nodes at the front of each mesh's node range in breadth-first order
 // (the root and the next two collapsed levels: the nodes every ray of the mesh
 // visits first); the trace kernels stage them in shared memory.
 constexpr int kTopNodes4 = 21;
-struct alignas(16) GNode4 {
-    float lmin[3], lmax[3];
-    float rmin[3], rmax[3];
-    float cmin[4][3];
-    float cmax[4][3];
+struct alignas(128) GNode4 {
+    float lo[3][4];
     uint32_t ref[4];
+    float hi[3][4];
+    uint32_t pad[4];
 };
+static_assert(sizeof(GNode4) == 128, "GNode4: lo and hi 64 bytes apart in a 128-byte line");
 
 // Triangle in leaf order: v0, e1 = v1 - v0, e2 = v2 - v0 (edges formed in double
 // as Triangle::_updateCache does, src/core/Hittables/Triangle.cpp:94-126).

@@ -916,12 +916,6 @@ ScenePack* pack_scene(const LuzSceneDesc* d)
                     const uint32_t qi = (uint32_t)S.nodes4.size();
                     S.nodes4.push_back(GNode4{});
                     GNode4 q{};
-                    for (int a = 0; a < 3; a++) {
-                        q.lmin[a] = b.lmin[a];
-                        q.lmax[a] = b.lmax[a];
-                        q.rmin[a] = b.rmin[a];
-                        q.rmax[a] = b.rmax[a];
-                    }
                     uint32_t sub[4] = {kEmptySlot, kEmptySlot, kEmptySlot, kEmptySlot};
                     for (int s = 0; s < 2; s++) {
                         const uint32_t c = s ? b.rref : b.lref;
@@ -931,10 +925,10 @@ ScenePack* pack_scene(const LuzSceneDesc* d)
                             q.ref[2 * s] = c;
                             q.ref[2 * s + 1] = kEmptySlot;
                             for (int a = 0; a < 3; a++) {
-                                q.cmin[2 * s][a] = cmn[a];
-                                q.cmax[2 * s][a] = cmx[a];
-                                q.cmin[2 * s + 1][a] = 0.f;
-                                q.cmax[2 * s + 1][a] = 0.f;
+                                q.lo[a][2 * s] = cmn[a];
+                                q.hi[a][2 * s] = cmx[a];
+                                q.lo[a][2 * s + 1] = kEmptyPlane;
+                                q.hi[a][2 * s + 1] = -kEmptyPlane;
                             }
                             continue;
                         }
@@ -942,8 +936,8 @@ ScenePack* pack_scene(const LuzSceneDesc* d)
                         for (int k = 0; k < 2; k++) {
                             const uint32_t gc = k ? cn.rref : cn.lref;
                             for (int a = 0; a < 3; a++) {
-                                q.cmin[2 * s + k][a] = k ? cn.rmin[a] : cn.lmin[a];
-                                q.cmax[2 * s + k][a] = k ? cn.rmax[a] : cn.lmax[a];
+                                q.lo[a][2 * s + k] = k ? cn.rmin[a] : cn.lmin[a];
+                                q.hi[a][2 * s + k] = k ? cn.rmax[a] : cn.lmax[a];
                             }
                             q.ref[2 * s + k] = gc;
                             if (!(gc & kLeafBit)) sub[2 * s + k] = gc;

@@ -1022,15 +1022,13 @@ static __device__ LUZ_LIGHT_ATTR F3 env_lookup_uv(const DScene& S, double u, dou
     v = clamp01d(v);
     const double x = (u * (double)E.width) - 0.5;
     const double y = ((1.0 - v) * (double)E.height) - 0.5;
-    const long long xf = (long long)floor(x), yf = (long long)floor(y);
-    auto wrap = [&](long long i) {
-        i %= (long long)E.width;
-        if (i < 0) i += E.width;
-        return (int)i;
-    };
+    // u and v lie in [0, 1], so floor(x) in [-1, width] and floor(y) in [-1, height - 1]: the
+    // index modulo the width is one conditional step either way (64-bit remainders are calls
+    // of about a hundred instructions each)
+    const int xf = min(max((int)floor(x), -1), E.width), yf = min(max((int)floor(y), -1), E.height - 1);
+    auto wrap = [&](int i) { return i < 0 ? i + E.width : (i >= E.width ? i - E.width : i); };
     const int x0 = wrap(xf), x1 = wrap(xf + 1);
-    const int y0 = (int)min(max(yf, 0ll), (long long)E.height - 1);
-    const int y1 = (int)min(max(yf + 1, 0ll), (long long)E.height - 1);
+    const int y0 = max(yf, 0), y1 = min(yf + 1, E.height - 1);
     const float tx = (float)(x - floor(x)), ty = (float)(y - floor(y));
     auto px = [&](int xx, int yy) {
         const float4 c = __ldg(S.env_texels + (size_t)yy * E.width + xx);
@@ -1193,7 +1191,16 @@ static __device__ LUZ_LIGHT_ATTR bool env_sample(const DScene& S, const Key& k, 
         else hi = mid;
     }
     if (lo >= n) lo = n - 1;
-    const int64_t y = lo / E.width, x = lo % E.width;
+    // 32-bit quotient where the texel count allows (a 64-bit one is a call)
+    int64_t y, x;
+    if (n <= (int64_t)0x7fffffff) {
+        const uint32_t q = (uint32_t)lo / (uint32_t)E.width;
+        y = q;
+        x = (int64_t)((uint32_t)lo - q * (uint32_t)E.width);
+    } else {
+        y = lo / E.width;
+        x = lo % E.width;
+    }
     const double u = ((double)x + (double)j.x) / (double)E.width;
     const double v = 1.0 - (((double)y + (double)j.y) / (double)E.height);
     const double phi = (wrap01d(u - (E.rotation / 360.0)) - 0.5) * 2.0 * kPiD;
@@ -1411,8 +1418,8 @@ static __device__ __noinline__ float light_pdf_value(const DScene& S, const GLig
         const TRay r = make_ray(origin, ray_dir_normalized(vec));
         float closest = kInf, u, v;
         int32_t slot;
-        LocalStack<true> st;
-        if (!mesh_closest<0u>(S, M, r, kTMin, closest, slot, u, v, -1, vs, st)) return 0.0f;
+        LocalStack st;
+        if (!mesh_closest<0u>(S, M, r, kTMin, closest, slot, u, v, -1, st)) return 0.0f;
         F3 n, gn;
         bool front;
         float tu, tv;
@@ -1429,7 +1436,7 @@ static __device__ __noinline__ float light_pdf_value(const DScene& S, const GLig
         const TRay r = make_ray(origin, ray_dir_normalized(vec));
         float closest = kInf;
         THit th{kInf, -1, 0, 0.f, 0.f};
-        LocalStack<true> st;
+        LocalStack st;
         object_closest<TF_ALL>(S, L.object, r, kTMin, closest, th, vs, st);
         if (th.obj < 0) return 0.0f;
         const Hit h = make_hit(S, r, th);

@@ -18,6 +18,13 @@ namespace {
 #define LUZ_SHADE_MIN_BLOCKS 6
 #endif
 
+#if LUZ_SHADE_BLOCK > 128
+#define LUZ_SHADE_SYNC __syncthreads();
+#define LUZ_SHADE_SKIP continue
+#else
+#define LUZ_SHADE_SYNC
+#define LUZ_SHADE_SKIP break
+#endif
 // Path of shade slot i: slots run through the class segments in class order.
 __device__ __forceinline__ uint32_t binned_path(const PathBuf& P, const uint32_t* bin, uint32_t i)
 {
@@ -30,15 +37,18 @@ __device__ __forceinline__ uint32_t binned_path(const PathBuf& P, const uint32_t
 }
 
 template <int MODE>
-__global__ void __launch_bounds__(kBlock, LUZ_SHADE_MIN_BLOCKS) k_shade(const DScene* __restrict__ Sp, WaveArgs w, PathBuf P, Ctrl* C, int bounce)
+__global__ void __launch_bounds__(kShadeBlock, LUZ_SHADE_MIN_BLOCKS) k_shade(const DScene* __restrict__ Sp, WaveArgs w, PathBuf P, Ctrl* C, int bounce)
 {
     const DScene& S = *Sp;
     const uint32_t count = C->count[bounce];
     const uint32_t* q = (bounce & 1) ? P.queue1 : P.queue0;
     uint32_t* nq = (bounce & 1) ? P.queue0 : P.queue1;
     const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-    const uint32_t wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    for (uint32_t base = wid * 32u; base < count; base += warps * 32u) {
+    const uint32_t wid = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+    for (uint32_t first = 0; first < count; first += warps * 32u) {
+        LUZ_SHADE_SYNC
+        const uint32_t base = first + wid * 32u;
+        if (base >= count) LUZ_SHADE_SKIP;
         const uint32_t i = base + lane_id();
         const bool valid = i < count;
         ShadeOut o;
@@ -67,7 +77,7 @@ __global__ void __launch_bounds__(kBlock, LUZ_SHADE_MIN_BLOCKS) k_shade(const DS
 
 // k_shade over a multi-scene wave: the scene and wave arguments are the path's segment's.
 template <int MODE>
-__global__ void __launch_bounds__(kBlock, LUZ_SHADE_MIN_BLOCKS) k_shade_batch(const DScene* __restrict__ scenes,
+__global__ void __launch_bounds__(kShadeBlock, LUZ_SHADE_MIN_BLOCKS) k_shade_batch(const DScene* __restrict__ scenes,
                                                                              const WaveArgs* __restrict__ segs,
                                                                              PathBuf P, Ctrl* C, int bounce)
 {
@@ -75,8 +85,11 @@ __global__ void __launch_bounds__(kBlock, LUZ_SHADE_MIN_BLOCKS) k_shade_batch(co
     const uint32_t* q = (bounce & 1) ? P.queue1 : P.queue0;
     uint32_t* nq = (bounce & 1) ? P.queue0 : P.queue1;
     const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-    const uint32_t wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    for (uint32_t base = wid * 32u; base < count; base += warps * 32u) {
+    const uint32_t wid = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+    for (uint32_t first = 0; first < count; first += warps * 32u) {
+        LUZ_SHADE_SYNC
+        const uint32_t base = first + wid * 32u;
+        if (base >= count) LUZ_SHADE_SKIP;
         const uint32_t i = base + lane_id();
         const bool valid = i < count;
         ShadeOut o;

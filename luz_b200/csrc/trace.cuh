@@ -74,15 +74,15 @@ enum ErrBits : uint32_t { ERR_TOP_STACK = 1u, ERR_MESH_STACK = 2u, ERR_CAUSTIC_G
 // memory (stage_top_nodes) and the mesh walks read them there.
 enum TraceFeature : uint32_t { TF_INSTANCE = 1u, TF_VOLUME = 2u, TF_ALL = 3u, TF_STAGED = 4u };
 
-// The staged nodes (kTopNodes4 x 160 B) of a trace kernel's block.
-static __shared__ float4 s_top4[kTopNodes4 * 10];
+// The staged nodes of a trace kernel's block.
+static __shared__ __align__(128) float4 s_top4[kTopNodes4 * 8];
 
 // Copies the staged node range into shared memory; every thread of the block calls it
 // once, before its first traversal.
 __device__ __forceinline__ void stage_top_nodes(const DScene& S)
 {
     const float4* src = reinterpret_cast<const float4*>(S.nodes4 + S.top4_base);
-    for (uint32_t i = threadIdx.x; i < S.top4_count * 10u; i += blockDim.x) s_top4[i] = __ldg(src + i);
+    for (uint32_t i = threadIdx.x; i < S.top4_count * 8u; i += blockDim.x) s_top4[i] = __ldg(src + i);
     __syncthreads();
 }
 
@@ -132,15 +132,11 @@ struct THit {
     float u, v;
 };
 
-// Per-ray traversal context: the volume distance sample (evaluated once, on
-// first use) and counts of the records read (mesh nodes, triangles, top-level
-// nodes/children/objects), used for the algorithmic-bytes roofline.
+// Per-ray traversal context: the volume distance sample (evaluated once, on first use).
 struct VolSample {
     const Key* key;
     double u;
     bool have;
-    uint32_t nodes = 0, tris = 0, top = 0;
-    uint32_t bnodes = 0;   // binary-tree node visits the collapsed walk stands for
     __device__ __forceinline__ double get()
     {
         if (!have) {
@@ -272,57 +268,155 @@ __device__ __forceinline__ GTri load_tri(const GTri* tris, uint32_t i)
     t.e2[0] = c.x; t.e2[1] = c.y; t.e2[2] = c.z; t.pad = 0;
     return t;
 }
-__device__ __forceinline__ GNode4 load_node4(const GNode4* nodes, uint32_t i)
+// Address of a collapsed node: the staged copy when it lies in the staged range, else
+// global memory (the same bytes either way).
+template <uint32_t F>
+__device__ __forceinline__ const char* node4_at(const DScene& S, uint32_t ref)
 {
-    const float4* p = reinterpret_cast<const float4*>(nodes + i);
-    float4 v[10];
-#pragma unroll
-    for (int k = 0; k < 10; k++) v[k] = ld4(p + k);
-    GNode4 n;
-    float* f = reinterpret_cast<float*>(&n);
-#pragma unroll
-    for (int k = 0; k < 10; k++) {
-        f[4 * k] = v[k].x;
-        f[4 * k + 1] = v[k].y;
-        f[4 * k + 2] = v[k].z;
-        f[4 * k + 3] = v[k].w;
+    if constexpr ((F & TF_STAGED) != 0) {
+        const uint32_t j = ref - S.top4_base;
+        if (j < S.top4_count) return reinterpret_cast<const char*>(s_top4 + 8 * j);
     }
-    return n;
+    return reinterpret_cast<const char*>(S.nodes4 + ref);
+}
+template <uint32_t F, class T>
+__device__ __forceinline__ T node4_ld(const char* p)
+{
+    if constexpr ((F & TF_STAGED) != 0) return *reinterpret_cast<const T*>(p);
+    else return __ldg(reinterpret_cast<const T*>(p));
 }
 
-// The entry part of a GNode4 (its four entry boxes and refs, without the two
-// side boxes): what the any-hit walk reads, seven of the ten 16-byte loads.
-struct GNode4C {
-    float cmin[4][3];
-    float cmax[4][3];
+// The four entry boxes of a collapsed node against a ray: which are met before tmax,
+// their entry distances and, for the visit order, those of the two sides (nl: slots 0
+// and 1, nr: slots 2 and 3; meaningful where the side holds an accepted entry).
+struct Node4Test {
+    bool ha[4];
+    float na[4];
+    float nl, nr;
+    bool hl, hr;   // SIDES: the side boxes themselves are met
     uint32_t ref[4];
 };
-static_assert(offsetof(GNode4, cmin) == 48 && offsetof(GNode4, ref) == 144 && sizeof(GNode4) == 160,
-              "GNode4 layout: the entry loads start at byte 48");
-static_assert(sizeof(GNode4C) == 112, "GNode4C is the last 112 bytes of a GNode4");
-__device__ __forceinline__ GNode4C load_node4_entries(const GNode4* nodes, uint32_t i)
+
+// FAST: the ray's sign picks each axis's near and far planes at the load, so that a box
+// costs six FMAs, a three-input max and min each with one more, and a comparison, with no
+// per-plane min / max: the fma is monotone in the plane, so near <= far as box_hit_fast's
+// min and max would order them. A side's entry distance follows from its slots' near
+// distances (the side's box is the union of its slots' boxes and the fma is monotone, so
+// its near distance along an axis is the smaller of the slots'): the same values as a test
+// of the stored side box, for five operations instead of eleven and three loads less.
+template <bool FAST, uint32_t F, bool ORDER, bool SIDES>
+__device__ __forceinline__ void node4_test(const DScene& S, uint32_t nref, const TRay& r, float tmax, Node4Test& T)
 {
-    const float4* p = reinterpret_cast<const float4*>(nodes + i) + 3;   // skips lmin..rmax (48 B)
-    float4 v[7];
+    const char* p = node4_at<F>(S, nref);
+    const uint4 rf = node4_ld<F, uint4>(p + 48);
+    T.ref[0] = rf.x;
+    T.ref[1] = rf.y;
+    T.ref[2] = rf.z;
+    T.ref[3] = rf.w;
+    if constexpr (FAST) {
+        const F3 noi = neg_o_inv(r);
+        const uint32_t sx = (__float_as_uint(r.inv.x) >> 31) << 6, sy = (__float_as_uint(r.inv.y) >> 31) << 6,
+                       sz = (__float_as_uint(r.inv.z) >> 31) << 6;
+        const float4 ax = node4_ld<F, float4>(p + sx), ay = node4_ld<F, float4>(p + 16 + sy),
+                     az = node4_ld<F, float4>(p + 32 + sz);
+        const float4 bx = node4_ld<F, float4>(p + (64u - sx)), by = node4_ld<F, float4>(p + 16 + (64u - sy)),
+                     bz = node4_ld<F, float4>(p + 32 + (64u - sz));
+        const float nx[4] = {fmaf(ax.x, r.inv.x, noi.x), fmaf(ax.y, r.inv.x, noi.x), fmaf(ax.z, r.inv.x, noi.x),
+                             fmaf(ax.w, r.inv.x, noi.x)};
+        const float ny[4] = {fmaf(ay.x, r.inv.y, noi.y), fmaf(ay.y, r.inv.y, noi.y), fmaf(ay.z, r.inv.y, noi.y),
+                             fmaf(ay.w, r.inv.y, noi.y)};
+        const float nz[4] = {fmaf(az.x, r.inv.z, noi.z), fmaf(az.y, r.inv.z, noi.z), fmaf(az.z, r.inv.z, noi.z),
+                             fmaf(az.w, r.inv.z, noi.z)};
+        const float fx[4] = {fmaf(bx.x, r.inv.x, noi.x), fmaf(bx.y, r.inv.x, noi.x), fmaf(bx.z, r.inv.x, noi.x),
+                             fmaf(bx.w, r.inv.x, noi.x)};
+        const float fy[4] = {fmaf(by.x, r.inv.y, noi.y), fmaf(by.y, r.inv.y, noi.y), fmaf(by.z, r.inv.y, noi.y),
+                             fmaf(by.w, r.inv.y, noi.y)};
+        const float fz[4] = {fmaf(bz.x, r.inv.z, noi.z), fmaf(bz.y, r.inv.z, noi.z), fmaf(bz.z, r.inv.z, noi.z),
+                             fmaf(bz.w, r.inv.z, noi.z)};
 #pragma unroll
-    for (int k = 0; k < 7; k++) v[k] = ld4(p + k);
-    GNode4C n;
-    float* f = reinterpret_cast<float*>(&n);
+        for (int k = 0; k < 4; k++) {
+            T.na[k] = fmax3f(fmaxf(kTMin, nx[k]), ny[k], nz[k]);
+            T.ha[k] = !(fmin3f(fminf(tmax, fx[k]), fy[k], fz[k]) <= T.na[k]);
+        }
+        if constexpr (ORDER) {
+            T.nl = fmax3f(fmaxf(kTMin, fminf(nx[0], nx[1])), fminf(ny[0], ny[1]), fminf(nz[0], nz[1]));
+            T.nr = fmax3f(fmaxf(kTMin, fminf(nx[2], nx[3])), fminf(ny[2], ny[3]), fminf(nz[2], nz[3]));
+        }
+        if constexpr (SIDES) {
+            T.hl = !(fmin3f(fminf(tmax, fmaxf(fx[0], fx[1])), fmaxf(fy[0], fy[1]), fmaxf(fz[0], fz[1])) <= T.nl);
+            T.hr = !(fmin3f(fminf(tmax, fmaxf(fx[2], fx[3])), fmaxf(fy[2], fy[3]), fmaxf(fz[2], fz[3])) <= T.nr);
+        }
+    } else {
+        const float4 lo[3] = {node4_ld<F, float4>(p), node4_ld<F, float4>(p + 16), node4_ld<F, float4>(p + 32)};
+        const float4 hi[3] = {node4_ld<F, float4>(p + 64), node4_ld<F, float4>(p + 80), node4_ld<F, float4>(p + 96)};
+        const float mn[4][3] = {{lo[0].x, lo[1].x, lo[2].x}, {lo[0].y, lo[1].y, lo[2].y},
+                                {lo[0].z, lo[1].z, lo[2].z}, {lo[0].w, lo[1].w, lo[2].w}};
+        const float mx[4][3] = {{hi[0].x, hi[1].x, hi[2].x}, {hi[0].y, hi[1].y, hi[2].y},
+                                {hi[0].z, hi[1].z, hi[2].z}, {hi[0].w, hi[1].w, hi[2].w}};
 #pragma unroll
-    for (int k = 0; k < 7; k++) {
-        f[4 * k] = v[k].x;
-        f[4 * k + 1] = v[k].y;
-        f[4 * k + 2] = v[k].z;
-        f[4 * k + 3] = v[k].w;
+        for (int k = 0; k < 4; k++) {
+            T.na[k] = 0.f;
+            T.ha[k] = T.ref[k] != kEmptySlot && box_hit(mn[k], mx[k], r, tmax, T.na[k]);
+        }
+        if constexpr (ORDER) {
+#pragma unroll
+            for (int s = 0; s < 2; s++) {
+                float umn[3], umx[3], n = 0.f;
+#pragma unroll
+                for (int a = 0; a < 3; a++) {
+                    umn[a] = fminf(mn[2 * s][a], mn[2 * s + 1][a]);
+                    umx[a] = fmaxf(mx[2 * s][a], mx[2 * s + 1][a]);
+                }
+                const bool h = box_hit(umn, umx, r, tmax, n);
+                if (s) {
+                    T.nr = n;
+                    T.hr = h;
+                } else {
+                    T.nl = n;
+                    T.hl = h;
+                }
+            }
+        }
     }
-    return n;
+}
+
+// The accepted entries of a collapsed node in visit order: the nearer side first (ties:
+// the right one), and on a side the nearer entry first (ties: the right one).
+struct Node4Order {
+    uint32_t ref[4];
+    float near[4];
+    bool on[4];   // first side's first, its second, the other side's first, its second
+};
+__device__ __forceinline__ void node4_order(const Node4Test& T, Node4Order& O)
+{
+    // second entry of a side first unless the first is accepted and strictly nearer
+    const bool lswap = T.ha[1] && !(T.ha[0] && T.na[0] < T.na[1]);
+    const bool rswap = T.ha[3] && !(T.ha[2] && T.na[2] < T.na[3]);
+    const bool l1 = T.ha[0] || T.ha[1], l2 = T.ha[0] && T.ha[1];
+    const bool r1 = T.ha[2] || T.ha[3], r2 = T.ha[2] && T.ha[3];
+    const bool rf = r1 && !(l1 && T.nl < T.nr);
+    const uint32_t la = lswap ? T.ref[1] : T.ref[0], lb = lswap ? T.ref[0] : T.ref[1];
+    const uint32_t ra = rswap ? T.ref[3] : T.ref[2], rb = rswap ? T.ref[2] : T.ref[3];
+    const float lan = lswap ? T.na[1] : T.na[0], lbn = lswap ? T.na[0] : T.na[1];
+    const float ran = rswap ? T.na[3] : T.na[2], rbn = rswap ? T.na[2] : T.na[3];
+    O.ref[0] = rf ? ra : la;
+    O.near[0] = rf ? ran : lan;
+    O.on[0] = l1 || r1;
+    O.ref[1] = rf ? rb : lb;
+    O.near[1] = rf ? rbn : lbn;
+    O.on[1] = rf ? r2 : l2;
+    O.ref[2] = rf ? la : ra;
+    O.near[2] = rf ? lan : ran;
+    O.on[2] = l1 && r1;
+    O.ref[3] = rf ? lb : rb;
+    O.near[3] = rf ? lbn : rbn;
+    O.on[3] = l1 && r1 && (rf ? l2 : r2);
 }
 
 // Visit order of a collapsed node's entries, as the binary near-first
 // traversal (Mesh::hit, Mesh.cpp:578-660) would reach them: the nearer of L
 // and R first (ties: R), and within each the nearer child first (ties: the
-// right one). mesh_closest_walk computes each accepted entry's position in
-// this order.
+// right one): node4_order.
 //
 // Testing all boxes at N's visit instead of at L's and R's gives the same
 // visits: L is visited right after N (nothing changes `closest` in between),
@@ -334,64 +428,24 @@ __device__ __forceinline__ GNode4C load_node4_entries(const GNode4* nodes, uint3
 // child is itself rejected.
 
 // Mesh traversal stack in the thread's local memory: node or leaf reference
-// and near distance per entry; NEAR = false drops the distances (any-hit never
-// prunes on them). (A variant holding the top 8-32 entries in a shared-memory
-// tile, one bank per thread, measured no faster on B200.)
-template <bool NEAR>
+// and near distance per entry.
 struct LocalStack {
     uint32_t r[kMeshStack4];
-    float n[NEAR ? kMeshStack4 : 1];
+    float n[kMeshStack4];
     __device__ __forceinline__ void set(int d, uint32_t ref, float near)
     {
         r[d] = ref;
-        if constexpr (NEAR) n[d] = near;
+        n[d] = near;
     }
     __device__ __forceinline__ uint32_t ref(int d) const { return r[d]; }
-    __device__ __forceinline__ float near(int d) const
-    {
-        if constexpr (NEAR) return n[d];
-        else return 0.0f;
-    }
+    __device__ __forceinline__ float near(int d) const { return n[d]; }
 };
-
-// A collapsed node from the staged copy when it lies in the staged range, else from
-// global memory (the same bytes either way).
-template <uint32_t F>
-__device__ __forceinline__ GNode4 fetch_node4(const DScene& S, uint32_t ref)
-{
-    if constexpr ((F & TF_STAGED) != 0) {
-        const uint32_t j = ref - S.top4_base;
-        if (j < S.top4_count) {
-            GNode4 n;
-            float4* d = reinterpret_cast<float4*>(&n);
-#pragma unroll
-            for (int k = 0; k < 10; k++) d[k] = s_top4[10 * j + k];
-            return n;
-        }
-    }
-    return load_node4(S.nodes4, ref);
-}
-template <uint32_t F>
-__device__ __forceinline__ GNode4C fetch_node4_entries(const DScene& S, uint32_t ref)
-{
-    if constexpr ((F & TF_STAGED) != 0) {
-        const uint32_t j = ref - S.top4_base;
-        if (j < S.top4_count) {
-            GNode4C n;
-            float4* d = reinterpret_cast<float4*>(&n);
-#pragma unroll
-            for (int k = 0; k < 7; k++) d[k] = s_top4[10 * j + 3 + k];
-            return n;
-        }
-    }
-    return load_node4_entries(S.nodes4, ref);
-}
 
 // Mesh::hit — closest triangle; closest is updated in place.
 template <bool FAST, uint32_t F, class Stk>
 __device__ __forceinline__ bool mesh_closest_walk(const DScene& S, const GMesh& M, const TRay& r, float tmin,
                                                   float& closest, int32_t& slot, float& bu, float& bv, int32_t skip,
-                                                  VolSample& vs, Stk& st)
+                                                  Stk& st)
 {
     float root_near;
     if (!mesh_box<FAST>(M.bmin, M.bmax, r, neg_o_inv(r), closest, root_near)) return false;
@@ -411,7 +465,6 @@ __device__ __forceinline__ bool mesh_closest_walk(const DScene& S, const GMesh& 
                 for (uint32_t i = first; i < first + cnt; i++) {
                     if ((int32_t)i == skip) continue;
                     const GTri T = load_tri(S.tris, i);
-                    vs.tris++;
                     float t, u, v;
                     if (tri_test(T, r, tmin, closest, t, u, v)) {
                         closest = t;
@@ -422,56 +475,21 @@ __device__ __forceinline__ bool mesh_closest_walk(const DScene& S, const GMesh& 
                     }
                 }
             } else {
-                const GNode4 n = fetch_node4<F>(S, ref);
-                vs.nodes++;
-                float nl = 0.f, nr = 0.f;
-                const F3 noi = FAST ? neg_o_inv(r) : F3{0.f, 0.f, 0.f};
-                const bool hl = mesh_box<FAST>(n.lmin, n.lmax, r, noi, closest, nl);
-                const bool hr = mesh_box<FAST>(n.rmin, n.rmax, r, noi, closest, nr);
-                bool ha[4];
-                float na[4];
-#pragma unroll
-                for (int k = 0; k < 4; k++) {
-                    na[k] = 0.f;
-                    ha[k] = n.ref[k] != kEmptySlot && mesh_box<FAST>(n.cmin[k], n.cmax[k], r, noi, closest, na[k]);
-                }
-                // node4_order's visit order as a position per accepted entry
-                // (side offset + place within the side), without appending to
-                // arrays. An accepted entry implies an accepted side box (the
-                // entry box lies inside it), so hl/hr only decide which side goes
-                // first when both hold entries: the nearer (ties: R).
-                const int cl = (int)ha[0] + (int)ha[1], cr = (int)ha[2] + (int)ha[3];
-                const bool r_first = (cl > 0 && cr > 0) ? !(nl < nr) : (cr > 0);
-                const int ne = cl + cr;
-                // binary-node visits this node stands for: N itself, and each accepted
-                // side that is an interior node (two entries) of the binary tree
-                vs.bnodes += 1u + (uint32_t)(hl && n.ref[1] != kEmptySlot) + (uint32_t)(hr && n.ref[3] != kEmptySlot);
+                Node4Test T;
+                node4_test<FAST, F, true, false>(S, ref, r, closest, T);
+                const int ne = (int)T.ha[0] + (int)T.ha[1] + (int)T.ha[2] + (int)T.ha[3];
                 if (sp + ne > S.mesh_stack_limit) {
                     atomicOr(S.error, ERR_MESH_STACK);
                     break;
                 }
                 if (ne > 0) {
-                    uint32_t first_ref = 0;
-                    float first_near = 0.f;
+                    Node4Order o;
+                    node4_order(T, o);
 #pragma unroll
-                    for (int k = 0; k < 4; k++) {
-                        const int side = k >> 1;
-                        const bool a_first = na[2 * side] < na[2 * side + 1];   // ties: the right entry first
-                        const bool behind_partner = ha[k ^ 1] && ((k & 1) ? a_first : !a_first);
-                        const bool side_second = side ? !r_first : r_first;
-                        const int pos = (side_second ? (side ? cl : cr) : 0) + (behind_partner ? 1 : 0);
-                        if (ha[k]) {
-                            if (pos == 0) {
-                                first_ref = n.ref[k];
-                                first_near = na[k];
-                            } else {
-                                st.set(sp + ne - 1 - pos, n.ref[k], na[k]);
-                            }
-                        }
-                    }
-                    sp += ne - 1;
-                    ref = first_ref;
-                    near = first_near;
+                    for (int k = 3; k > 0; k--)
+                        if (o.on[k]) st.set(sp++, o.ref[k], o.near[k]);
+                    ref = o.ref[0];
+                    near = o.near[0];
                     continue;
                 }
             }
@@ -486,95 +504,10 @@ __device__ __forceinline__ bool mesh_closest_walk(const DScene& S, const GMesh& 
 
 template <uint32_t F, class Stk>
 __device__ __forceinline__ bool mesh_closest(const DScene& S, const GMesh& M, const TRay& r, float tmin, float& closest,
-                                             int32_t& slot, float& bu, float& bv, int32_t skip, VolSample& vs, Stk& st)
+                                             int32_t& slot, float& bu, float& bv, int32_t skip, Stk& st)
 {
-    if (mesh_fast_slabs(M, r)) return mesh_closest_walk<true, F>(S, M, r, tmin, closest, slot, bu, bv, skip, vs, st);
-    return mesh_closest_walk<false, F>(S, M, r, tmin, closest, slot, bu, bv, skip, vs, st);
-}
-
-// Mesh::hitAny
-template <bool FAST, uint32_t F, class Stk>
-__device__ __forceinline__ bool mesh_any_walk(const DScene& S, const GMesh& M, const TRay& r, float tmin, float tmax,
-                                              int32_t skip, VolSample& vs, Stk& st)
-{
-    float root_near;
-    if (!mesh_box<FAST>(M.bmin, M.bmax, r, neg_o_inv(r), tmax, root_near)) return false;
-    // The walk of mesh_closest without pruning: any accepted entry may hold an
-    // occluder and the first one found ends the walk, so the entries of a node are
-    // taken in a fixed order (left side, then right) instead of nearest first; the
-    // answer does not depend on the order.
-    uint32_t ref = (uint32_t)M.root4_ref;
-    int sp = 0;
-    bool hit = false;
-    while (true) {
-        if (ref & kLeafBit) {
-            const uint32_t first = (ref & 0x7fffffffu) >> 3;
-            const uint32_t cnt = (ref & 7u) + 1u;
-            for (uint32_t i = first; i < first + cnt; i++) {
-                if ((int32_t)i == skip) continue;
-                const GTri T = load_tri(S.tris, i);
-                vs.tris++;
-                float t, u, v;
-                if (tri_test(T, r, tmin, tmax, t, u, v)) {
-                    hit = true;
-                    break;
-                }
-            }
-            if (hit) break;
-        } else {
-            // Only the four entry boxes are tested. The two side boxes would
-            // reject nothing more: an entry box lies inside its side's box (both
-            // rounded outward from nested FP64 boxes), and every slab form here is
-            // monotone in the plane coordinate, so a ray that misses a side box
-            // misses the entry boxes inside it. The triangles tested, and so the
-            // answer, are the same as with the side tests.
-            const GNode4C n = fetch_node4_entries<F>(S, ref);
-            vs.nodes++;
-            const F3 noi = FAST ? neg_o_inv(r) : F3{0.f, 0.f, 0.f};
-            bool ha[4];
-#pragma unroll
-            for (int k = 0; k < 4; k++) {
-                float na;
-                ha[k] = n.ref[k] != kEmptySlot && mesh_box<FAST>(n.cmin[k], n.cmax[k], r, noi, tmax, na);
-            }
-            // Entries in slot order; an entry's place is the number of accepted
-            // entries before it (selects, no running index into an array).
-            const int ne = (int)ha[0] + (int)ha[1] + (int)ha[2] + (int)ha[3];
-            // binary-node visits: N, and each interior side with an accepted entry
-            vs.bnodes += 1u + (uint32_t)(n.ref[1] != kEmptySlot && (ha[0] || ha[1]))
-                         + (uint32_t)(n.ref[3] != kEmptySlot && (ha[2] || ha[3]));
-            if (sp + ne > S.mesh_stack_limit) {
-                atomicOr(S.error, ERR_MESH_STACK);
-                break;
-            }
-            if (ne > 0) {
-                uint32_t first_ref = 0;
-                int pos = 0;
-#pragma unroll
-                for (int k = 0; k < 4; k++) {
-                    if (ha[k]) {
-                        if (pos == 0) first_ref = n.ref[k];
-                        else st.set(sp + ne - 1 - pos, n.ref[k], 0.f);
-                        pos++;
-                    }
-                }
-                sp += ne - 1;
-                ref = first_ref;
-                continue;
-            }
-        }
-        if (sp == 0) break;
-        ref = st.ref(--sp);
-    }
-    return hit;
-}
-
-template <uint32_t F, class Stk>
-__device__ __forceinline__ bool mesh_any(const DScene& S, const GMesh& M, const TRay& r, float tmin, float tmax,
-                                         int32_t skip, VolSample& vs, Stk& st)
-{
-    if (mesh_fast_slabs(M, r)) return mesh_any_walk<true, F>(S, M, r, tmin, tmax, skip, vs, st);
-    return mesh_any_walk<false, F>(S, M, r, tmin, tmax, skip, vs, st);
+    if (mesh_fast_slabs(M, r)) return mesh_closest_walk<true, F>(S, M, r, tmin, closest, slot, bu, bv, skip, st);
+    return mesh_closest_walk<false, F>(S, M, r, tmin, closest, slot, bu, bv, skip, st);
 }
 
 // Rectangle::hit geometric test (Rectangle.cpp:212-249); returns t.
@@ -719,7 +652,8 @@ static __device__ float volume_overlap(const GObject& O, F3 o, F3 d, float tmin,
     return (exit - entry) * sqrtf(len2(d));
 }
 
-static __device__ bool volume_distance(const GObject& O, const TRay& r, float tmin, float tmax, VolSample& vs, float& t)
+template <class VS>
+__device__ bool volume_distance(const GObject& O, const TRay& r, float tmin, float tmax, VS& vs, float& t)
 {
     float entry, exit;
     if (O.aux == 3 /* LUZ_OBJ_CUBE */) {
@@ -783,7 +717,6 @@ __device__ __forceinline__ void object_closest(const DScene& S, int32_t oi, cons
                                                THit& h, VolSample& vs, Stk& st)
 {
     const GObject O = S.objects[oi];
-    vs.top++;
     const bool src = oi == r.xobj;
     float t;
     switch (O.kind) {
@@ -815,7 +748,7 @@ __device__ __forceinline__ void object_closest(const DScene& S, int32_t oi, cons
     case OK_MESH: {
         int32_t slot;
         float u, v;
-        if (mesh_closest<F>(S, S.meshes[O.aux], r, tmin, closest, slot, u, v, src ? r.xprim : -1, vs, st))
+        if (mesh_closest<F>(S, S.meshes[O.aux], r, tmin, closest, slot, u, v, src ? r.xprim : -1, st))
             h = THit{closest, oi, slot, u, v};
         break;
     }
@@ -827,7 +760,7 @@ __device__ __forceinline__ void object_closest(const DScene& S, int32_t oi, cons
         float lc = closest * s;
         int32_t slot;
         float u, v;
-        if (!mesh_closest<F>(S, S.meshes[O.aux], lr, tmin * s, lc, slot, u, v, src ? r.xprim : -1, vs, st)) break;
+        if (!mesh_closest<F>(S, S.meshes[O.aux], lr, tmin * s, lc, slot, u, v, src ? r.xprim : -1, st)) break;
         const float wt = lc / s;
         if (!isfinite(wt) || wt < tmin || wt > closest) break;
         closest = wt;
@@ -843,42 +776,6 @@ __device__ __forceinline__ void object_closest(const DScene& S, int32_t oi, cons
         break;
     default:
         break;
-    }
-}
-
-template <uint32_t F, class Stk>
-__device__ __forceinline__ bool object_any(const DScene& S, int32_t oi, const TRay& r, float tmin, float tmax, VolSample& vs,
-                                           Stk& st)
-{
-    const GObject O = S.objects[oi];
-    vs.top++;
-    const bool src = oi == r.xobj;
-    float t;
-    switch (O.kind) {
-    case OK_RECT:
-        return !src && rect_test(S.rects[O.aux], r, tmin, tmax, t);
-    case OK_CUBE:
-        for (int f = 0; f < 6; f++)
-            if (!(src && f == r.xprim) && rect_test(S.rects[O.aux + f], r, tmin, tmax, t)) return true;
-        return false;
-    case OK_SPHERE:
-        return sphere_test(O, r, tmin, tmax, t, src);
-    case OK_PLANE:
-        return !src && plane_test(O, r, tmin, tmax, t);
-    case OK_MESH:
-        return mesh_any<F>(S, S.meshes[O.aux], r, tmin, tmax, src ? r.xprim : -1, vs, st);
-    case OK_INSTANCE: {
-        if constexpr (!(F & TF_INSTANCE)) return false;
-        TRay lr;
-        float s;
-        if (!local_ray(O, r, lr, s)) return false;
-        return mesh_any<F>(S, S.meshes[O.aux], lr, tmin * s, tmax * s, src ? r.xprim : -1, vs, st);
-    }
-    case OK_VOLUME:
-        if constexpr (!(F & TF_VOLUME)) return false;
-        return volume_distance(O, r, tmin, tmax, vs, t);
-    default:
-        return false;
     }
 }
 
@@ -921,7 +818,6 @@ __device__ __forceinline__ THit closest_hit(const DScene& S, const TRay& r, floa
                 continue;
             }
             const GTopNode N = S.top_nodes[idx];
-            vs.top += 1 + (uint32_t)N.child_count;
             float dummy;
             if (kind == 1) {
                 if (!box_hit(N.bmin, N.bmax, r, closest, dummy)) continue;
@@ -979,54 +875,6 @@ __device__ __forceinline__ THit closest_hit(const DScene& S, const TRay& r, floa
     for (int i = 0; i < S.k.unaccel_count; i++)
         object_closest<F>(S, S.index_pool[S.k.unaccel_offset + i], r, tmin, closest, h, vs, st);
     return h;
-}
-
-// isShadowOccluded body with explicit [tmin, tmax] (tmax <= T_MIN -> not occluded).
-template <uint32_t F, class Stk>
-__device__ __forceinline__ bool any_hit(const DScene& S, const TRay& r, float tmin, float tmax, VolSample& vs, Stk& st)
-{
-    if (tmax <= kTMin) return false;
-    bool occ = false;
-    if (S.k.accel_kind == 2) {
-        occ = object_any<F>(S, S.k.accel_object, r, tmin, tmax, vs, st);
-    } else if (S.k.accel_kind == 1) {
-        uint32_t sref[kTopStack];
-        float snear[kTopStack];
-        int sp = 0;
-        TOP_PUSH(0, 1, 0.f);
-        while (sp > 0) {
-            sp--;
-            const uint32_t e = sref[sp];
-            const uint32_t kind = e >> 30;
-            const int32_t idx = (int32_t)(e & 0x3fffffffu);
-            if (kind >= 2) {
-                if (object_any<F>(S, idx, r, tmin, tmax, vs, st)) {
-                    occ = true;
-                    break;
-                }
-                continue;
-            }
-            const GTopNode N = S.top_nodes[idx];
-            vs.top += 1 + (uint32_t)N.child_count;
-            float dummy;
-            if (kind == 1 && !box_hit(N.bmin, N.bmax, r, tmax, dummy)) continue;
-            const int n = N.child_count;
-            const GTopChild* C = S.top_children + N.child_start;
-            const bool test_kids = !(n != 2 && n <= 3);
-            for (int i = n - 1; i >= 0; i--) {
-                if (test_kids) {
-                    float cn;
-                    if (!box_hit(C[i].bmin, C[i].bmax, r, tmax, cn)) continue;
-                    TOP_PUSH(C[i].ref, C[i].is_node ? 1 : 3, 0.f);
-                } else {
-                    TOP_PUSH(C[i].ref, C[i].is_node ? 1 : 3, 0.f);
-                }
-            }
-        }
-    }
-    for (int i = 0; i < S.k.unaccel_count && !occ; i++)
-        occ = object_any<F>(S, S.index_pool[S.k.unaccel_offset + i], r, tmin, tmax, vs, st);
-    return occ;
 }
 
 }  // namespace luz

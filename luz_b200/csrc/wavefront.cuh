@@ -9,6 +9,10 @@ namespace luz {
 
 constexpr int kMaxBounceSlots = 256;
 constexpr int kBlock = 128;
+#ifndef LUZ_SHADE_BLOCK
+#define LUZ_SHADE_BLOCK 128
+#endif
+constexpr int kShadeBlock = LUZ_SHADE_BLOCK;   // threads per block of the shade kernels
 constexpr int kShadeClasses = 10;           // 0 = miss, 1..9 = material type of the hit
 
 struct Ctrl {
@@ -289,7 +293,7 @@ static __device__ __noinline__ void relocate_subsurface(const DScene& S, const G
     const float probe = fmaxf(radius + (4.0f * dl / mpu), 16.0f * kTMin);
     const TRay pr = make_ray(cand + n * probe, ray_dir_normalized(n * -1.0f));
     VolSample vs{&k, 0.0, false};
-    LocalStack<true> st;
+    LocalStack st;
     const THit th = closest_hit<TF_ALL>(S, pr, kTMin, kInf, vs, st);
     if (th.obj < 0) return;
     const Hit eh = make_hit(S, pr, th);
