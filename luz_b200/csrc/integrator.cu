@@ -48,13 +48,8 @@ __global__ void __launch_bounds__(kBlock) k_raygen(WaveArgs w, PathBuf P, Ctrl* 
     camera_ray(w, x, y, s, o, d);
     P.ray_o[p] = make_float4((float)o[0], (float)o[1], (float)o[2], __int_as_float(-1));
     P.ray_d[p] = make_float4((float)d[0], (float)d[1], (float)d[2], __int_as_float(-1));
-    P.thr[p] = make_float4(1.f, 1.f, 1.f, 0.f);
-    P.rad[p] = make_float4(0.f, 0.f, 0.f, __uint_as_float(PF_PREV_SPECULAR));
-    P.pend0[p] = make_float4(0.f, 0.f, 0.f, 0.f);
-    P.pend1[p] = make_float4(0.f, 0.f, 0.f, 0.f);
     P.pixel[p] = y * (uint32_t)w.width + x;
     P.sample[p] = s;
-    P.queue0[p] = (uint32_t)p;
 }
 
 // ---------------------------------------------------------------------------- trace (closest and any hits)
@@ -144,12 +139,13 @@ __device__ __forceinline__ void trace_extension(const DScene& S, const WaveArgs&
     Walk<F, false, COUNT, PathVolume> walk;
     walk.st = st;
     const uint32_t count = C->count[bounce], per = rays_per_fetch(count);
-    const uint32_t* q = (w.sorted_queue && bounce >= 1) ? w.sorted_queue : ((bounce & 1) ? P.queue1 : P.queue0);
+    // the first bounce's queue is the paths in order
+    const uint32_t* q = bounce == 0 ? nullptr : w.sorted_queue ? w.sorted_queue : ((bounce & 1) ? P.queue1 : P.queue0);
     while (true) {
         const uint32_t base = fetch_rays(&C->fetch_ext[bounce], per);
         if (base >= count) break;
         const bool valid = lane_id() < per && base + lane_id() < count;
-        const uint32_t p = valid ? q[base + lane_id()] : 0u;
+        const uint32_t p = !valid ? 0u : q ? q[base + lane_id()] : base + lane_id();
         walk.state = WS_DONE;
         if (valid) {
             const float4 o = P.ray_o[p], d = P.ray_d[p];
@@ -374,14 +370,9 @@ __global__ void __launch_bounds__(kBlock) k_raygen_batch(const WaveArgs* segs, c
     camera_ray(w, x, y, s, o, d);
     P.ray_o[p] = make_float4((float)o[0], (float)o[1], (float)o[2], __int_as_float(-1));
     P.ray_d[p] = make_float4((float)d[0], (float)d[1], (float)d[2], __int_as_float(-1));
-    P.thr[p] = make_float4(1.f, 1.f, 1.f, 0.f);
-    P.rad[p] = make_float4(0.f, 0.f, 0.f, __uint_as_float(PF_PREV_SPECULAR));
-    P.pend0[p] = make_float4(0.f, 0.f, 0.f, 0.f);
-    P.pend1[p] = make_float4(0.f, 0.f, 0.f, 0.f);
     P.pixel[p] = y * (uint32_t)w.width + x;
     P.sample[p] = s;
     P.seg[p] = sg;
-    P.queue0[p] = (uint32_t)p;
 }
 
 // One per-scene counter add per group of lanes with the same scene.
@@ -398,12 +389,13 @@ __device__ __forceinline__ void trace_extension_batch(const DScene* __restrict__
     Walk<TF_ALL, false, false, PathVolume> walk;
     walk.st = st;
     const uint32_t count = C->count[bounce], per = rays_per_fetch(count);
-    const uint32_t* q = (bounce & 1) ? P.queue1 : P.queue0;
+    const uint32_t* q = bounce == 0 ? nullptr : (bounce & 1) ? P.queue1 : P.queue0;
     while (true) {
         const uint32_t base = fetch_rays(&C->fetch_ext[bounce], per);
         if (base >= count) break;
         const bool valid = lane_id() < per && base + lane_id() < count;
-        const uint32_t p = q[valid ? base + lane_id() : base];
+        const uint32_t at = valid ? base + lane_id() : base;
+        const uint32_t p = q ? q[at] : at;
         const WaveArgs& w = segs[P.seg[p]];
         const DScene& S = scenes[w.batch_scene];
         walk.state = WS_DONE;
@@ -1035,7 +1027,7 @@ struct luz_gpu_scene {
     // content (version changes with texels or the caustic map)
     std::vector<std::pair<std::size_t, std::size_t>> arena_fields;
     uint64_t uid = 0, version = 0;
-    ShadeKernel shade = nullptr;
+    bool shade_cold = false;         // the scene needs the shade kernels' cold code (set at creation)
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     // caustic photon map: buffers grown on demand; the map is kept while the
     // render seed and bounce limit stay the same (textures unchanged)
@@ -1215,6 +1207,20 @@ PathBuf lane_view(const PathBuf& b, int64_t off)
 
 namespace {
 
+// Shade kernel mode of a scene's plain renders.
+int shade_mode(const luz_gpu_scene* s) { return s->pack->consts.caustics.enabled ? 1 : 0; }
+
+// Whether a scene holds what the shade kernels' cold code serves: Principled materials (with
+// their subsurface relocation), roughness textures, emissive meshes and instances, IES
+// profiles, cube-cross spheres, the atmosphere.
+bool shade_cold(const ScenePack& P)
+{
+    bool cold = P.consts.sky == 2 || P.consts.cube_cross_spheres != 0;
+    for (const GMaterial& m : P.materials) cold |= m.type == MT_PRINCIPLED || m.rtexture >= 0;
+    for (const GLight& l : P.lights) cold |= l.kind == LK_MESH || l.kind == LK_INSTANCE || l.ies >= 0;
+    return cold;
+}
+
 // Smallest lane of a two-lane render (render_prepare).
 constexpr int64_t kMinLanePaths = int64_t(1) << 22;
 
@@ -1258,9 +1264,15 @@ struct StageTimer {
     }
 };
 
-// shade: the shade instantiation to run (NULL: the scene's own).
-void launch_bounces(luz_gpu_scene* s, const WaveArgs& w, cudaStream_t st, int64_t& launches, StageTimer& T,
-                    ShadeKernel shade, const PathBuf& pb, Ctrl* ctrl)
+// Waves from this many paths on shade the missed paths in a launch of their own: a second
+// launch per bounce against a leaner kernel for half of the vertices. Shade stage, one
+// launch / two: Cornell box (4.5 M paths) 2.15 / 2.03 ms, spheres under the sky (1.4 M) 0.53
+// / 0.57 ms, 640x360 draft (0.9 M) 0.80 / 0.84 ms, 96x64 preview 0.34 / 0.37 ms.
+constexpr int64_t kSplitShadePaths = int64_t(1) << 21;
+
+// mode: the shade kernel's (shade_mode(s), 2 or 3).
+void launch_bounces(luz_gpu_scene* s, const WaveArgs& w, cudaStream_t st, int64_t& launches, StageTimer& T, int mode,
+                    const PathBuf& pb, Ctrl* ctrl)
 {
     auto blocks = [](int tuned, int occ) { return tuned > 0 ? std::min(tuned, occ) : occ; };
     // no more blocks than the wave's rays could keep busy
@@ -1271,7 +1283,11 @@ void launch_bounces(luz_gpu_scene* s, const WaveArgs& w, cudaStream_t st, int64_
     const unsigned g_ext = grid(blocks(s->tune.extend_blocks_per_sm, s->occ_trace), 32);
     const unsigned g_sh = grid(blocks(s->tune.shadow_blocks_per_sm, s->occ_trace), 64);
     const unsigned g_shade = grid(blocks(s->tune.shade_blocks_per_sm, s->occ_shade), 1);
-    if (!shade) shade = s->shade;
+    const bool cold = s->shade_cold || w.nfor;
+    const bool split = mode < 2 && w.n >= kSplitShadePaths;
+    const ShadeKernel shade = shade_kernel(mode, split ? SHADE_HITS : SHADE_ALL, cold);
+    const ShadeKernel shade_misses = shade_kernel(mode, SHADE_MISSES, cold);
+    const unsigned g_miss = grid(16, 1);
     const int count = s->ds.counters ? 1 : 0;   // LUZ_RENDER_COUNT renders run the counting instantiations
     const uint32_t kv = (s->ds.k.features & TF_ALL) | (s->tune.staged_top_nodes && s->ds.top4_count ? TF_STAGED : 0u);
     const TraceKernel trace = kTraceKernels[count][kv];
@@ -1306,7 +1322,11 @@ void launch_bounces(luz_gpu_scene* s, const WaveArgs& w, cudaStream_t st, int64_
         launches++;
         if (!ext) break;
         T.mark(st, 1, true);
-        shade<<<g_shade, kShadeBlock, 0, st>>>(s->dds, w, pb, ctrl, b);
+        if (split) {
+            shade_misses<<<g_miss, kBlock, 0, st>>>(s->dds, w, pb, ctrl, b);
+            launches++;
+        }
+        shade<<<g_shade, kBlock, 0, st>>>(s->dds, w, pb, ctrl, b);
         T.mark(st, 1, false);
         launches++;
     }
@@ -1560,7 +1580,7 @@ void render_enqueue(RenderJob& J)
             w.list_mode = 0;
             CK(cudaMemsetAsync(lane_ctrl[L], 0, sizeof(Ctrl), ls));
             k_raygen<<<(unsigned)((w.n + kBlock - 1) / kBlock), kBlock, 0, ls>>>(w, lane_pb[L], lane_ctrl[L]);
-            launch_bounces(s, w, ls, J.launches, J.T, nullptr, lane_pb[L], lane_ctrl[L]);
+            launch_bounces(s, w, ls, J.launches, J.T, shade_mode(s), lane_pb[L], lane_ctrl[L]);
             // the film adds waves in order (samples of a pixel in sample order), the totals one at a time
             if (two && k > 0) CK(cudaStreamWaitEvent(ls, s->lane_acc[1 - L], 0));
             k_accumulate<<<(unsigned)((pc + 127) / 128), 128, 0, ls>>>(w, lane_pb[L], s->film);
@@ -1802,7 +1822,7 @@ int do_render_ex(luz_gpu_scene* s, const LuzRenderParams* p, const LuzAdaptivePa
                 w.list_mode = 0;
                 CK(cudaMemsetAsync(s->ctrl, 0, sizeof(Ctrl), st));
                 k_raygen<<<(unsigned)((w.n + kBlock - 1) / kBlock), kBlock, 0, st>>>(w, s->pb, s->ctrl);
-                launch_bounces(s, w, st, launches, T, nullptr, s->pb, s->ctrl);
+                launch_bounces(s, w, st, launches, T, shade_mode(s), s->pb, s->ctrl);
                 k_accumulate_px<<<(unsigned)((pc + 127) / 128), 128, 0, st>>>(w, s->pb, acc, nf);
                 k_tally<<<1, 1, 0, st>>>(s->ctrl, w.max_bounces, s->totals);
                 launches += 3;
@@ -1961,7 +1981,7 @@ int do_adjoint_backward(luz_gpu_scene* s, const LuzRenderParams* p, int32_t text
                 CK(cudaMemsetAsync(s->ctrl, 0, sizeof(Ctrl), st));
                 if (pass == 1 && rough) CK(cudaMemsetAsync(w.adj_rough, 0, sizeof(AdjRough) * (std::size_t)w.n, st));
                 k_raygen<<<grid, kBlock, 0, st>>>(w, s->pb, s->ctrl);
-                launch_bounces(s, w, st, launches, T0, shade_kernel(3), s->pb, s->ctrl);
+                launch_bounces(s, w, st, launches, T0, 3, s->pb, s->ctrl);
                 launches++;
                 if (pass == 0) {
                     k_path_color<<<grid, kBlock, 0, st>>>(w, s->pb);
@@ -2039,7 +2059,7 @@ int do_adjoint_emission(luz_gpu_scene* s, const LuzRenderParams* p, const float*
             CK(cudaMemsetAsync(s->ctrl, 0, sizeof(Ctrl), st));
             CK(cudaMemsetAsync(w.pend_light, 0xff, sizeof(int32_t) * (std::size_t)w.n, st));
             k_raygen<<<grid, kBlock, 0, st>>>(w, s->pb, s->ctrl);
-            launch_bounces(s, w, st, launches, T0, shade_kernel(3), s->pb, s->ctrl);
+            launch_bounces(s, w, st, launches, T0, 3, s->pb, s->ctrl);
             k_adjoint_emission_finish<<<grid, kBlock, 0, st>>>(s->ds, w, s->pb);
             launches += 2;
             waves++;
@@ -2121,7 +2141,7 @@ int do_adjoint_density(luz_gpu_scene* s, const LuzRenderParams* p, int32_t objec
             CK(cudaMemsetAsync(s->ctrl, 0, sizeof(Ctrl), st));
             CK(cudaMemsetAsync(w.dens_score, 0, sizeof(float2) * (std::size_t)w.n, st));
             k_raygen<<<grid, kBlock, 0, st>>>(w, s->pb, s->ctrl);
-            launch_bounces(s, w, st, launches, T0, shade_kernel(3), s->pb, s->ctrl);
+            launch_bounces(s, w, st, launches, T0, 3, s->pb, s->ctrl);
             k_adjoint_density_finish<<<grid, kBlock, 0, st>>>(s->ds, w, s->pb);
             launches += 2;
             waves++;
@@ -2357,11 +2377,11 @@ std::vector<std::vector<WaveArgs>> batch_waves(luz_gpu_scene* const* scenes, con
 // into a graph: every kernel reads the wave's size from device memory.
 cudaGraphExec_t batch_graph(BatchContext& C, const BatchWaveHeader* hdr, int max_b, int64_t cap_paths,
                             int64_t max_pix, int64_t max_segs, double* const* d_films, unsigned long long* d_rays,
-                            int32_t count, bool caustics, int sms, int occ_trace, int occ_shade,
+                            int32_t count, bool caustics, bool cold, int sms, int occ_trace, int occ_shade,
                             int64_t& launches)
 {
     (void)hdr;
-    const BatchShadeKernel shade = batch_shade_kernel(caustics ? 1 : 0);
+    const BatchShadeKernel shade = batch_shade_kernel(caustics ? 1 : 0, cold);
     cudaGraph_t g = nullptr;
     CK(cudaStreamBeginCapture(C.st, cudaStreamCaptureModeThreadLocal));
     try {
@@ -2374,7 +2394,7 @@ cudaGraphExec_t batch_graph(BatchContext& C, const BatchWaveHeader* hdr, int max
                                                                d_rays, d_rays + count);
             launches++;
             if (b > max_b) break;
-            shade<<<sms * occ_shade, kShadeBlock, 0, C.st>>>(C.d_scenes, C.d_segs, C.pb, C.ctrl, b);
+            shade<<<sms * occ_shade, kBlock, 0, C.st>>>(C.d_scenes, C.d_segs, C.pb, C.ctrl, b);
             launches++;
         }
         dim3 ag((unsigned)((max_pix + 127) / 128), (unsigned)max_segs);
@@ -2401,7 +2421,7 @@ int batch_render(luz_gpu_scene* const* scenes, const LuzRenderParams* params, in
     BatchContext& C = batch_context(device);
     std::lock_guard<std::mutex> lock(C.mu);
     CK(cudaSetDevice(device));
-    bool caustics = false;
+    bool caustics = false, cold = false;
     int max_b = 0;
     int64_t max_pix = 0, max_spp = 0;
     for (int32_t i = 0; i < count; i++) {   // photon maps are built per scene before the arena copy
@@ -2409,6 +2429,7 @@ int batch_render(luz_gpu_scene* const* scenes, const LuzRenderParams* params, in
         prepare_caustics(scenes[i], &params[i], scenes[i]->stream);
         CK(cudaStreamSynchronize(scenes[i]->stream));
         caustics |= scenes[i]->pack->consts.caustics.enabled != 0;
+        cold |= scenes[i]->shade_cold;
         max_b = std::max(max_b, params[i].max_bounces);
         max_pix = std::max<int64_t>(max_pix, (int64_t)params[i].width * params[i].height);
         max_spp = std::max<int64_t>(max_spp, params[i].spp);
@@ -2448,7 +2469,7 @@ int batch_render(luz_gpu_scene* const* scenes, const LuzRenderParams* params, in
     }
     int occ_trace = 1, occ_shade = 1;
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_trace, k_trace_batch, kBlock, 0));
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_shade, batch_shade_kernel(caustics ? 1 : 0), kShadeBlock, 0));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_shade, batch_shade_kernel(caustics ? 1 : 0, cold), kBlock, 0));
     occ_trace = std::max(1, occ_trace);
     occ_shade = std::max(1, occ_shade);
     const int sms = scenes[0]->sms;
@@ -2480,7 +2501,7 @@ int batch_render(luz_gpu_scene* const* scenes, const LuzRenderParams* params, in
             segs_max = std::max<int64_t>(segs_max, (int64_t)wv.size());
             for (const WaveArgs& w : wv) pix_max = std::max<int64_t>(pix_max, w.pix_count);
         }
-        cudaGraphExec_t ex = batch_graph(C, hdr, max_b, wave_max, pix_max, segs_max, d_films, d_rays, count, caustics,
+        cudaGraphExec_t ex = batch_graph(C, hdr, max_b, wave_max, pix_max, segs_max, d_films, d_rays, count, caustics, cold,
                                          sms, occ_trace, occ_shade, launches);
         CK(cudaMemsetAsync(films, 0, sizeof(double) * (std::size_t)film_doubles, st));
         CK(cudaMemsetAsync(d_rays, 0, sizeof(unsigned long long) * 2 * (std::size_t)count, st));
@@ -2685,7 +2706,7 @@ int do_render_noalloc(luz_gpu_scene* s, const LuzRenderParams* p, float* d_out, 
             w.list_mode = 0;
             CK(cudaMemsetAsync(A.ctrl, 0, sizeof(Ctrl), st));
             k_raygen<<<(unsigned)((w.n + kBlock - 1) / kBlock), kBlock, 0, st>>>(w, A.pb, A.ctrl);
-            launch_bounces(s, w, st, launches, T, nullptr, A.pb, A.ctrl);
+            launch_bounces(s, w, st, launches, T, shade_mode(s), A.pb, A.ctrl);
             k_accumulate<<<(unsigned)((pc + 127) / 128), 128, 0, st>>>(w, A.pb, A.film);
             k_tally<<<1, 1, 0, st>>>(A.ctrl, w.max_bounces, A.totals);
             launches += 3;
@@ -2819,8 +2840,9 @@ int luz_gpu_scene_create(const LuzSceneDesc* desc, int32_t device, luz_gpu_scene
         s->sms = prop.multiProcessorCount;
         const int feat = P.consts.features & TF_ALL;
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&s->occ_trace, kTraceKernels[0][feat], kBlock, 0));
-        s->shade = shade_kernel(P.consts.caustics.enabled ? 1 : 0);
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&s->occ_shade, s->shade, kShadeBlock, 0));
+        s->shade_cold = shade_cold(P);
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&s->occ_shade, shade_kernel(shade_mode(s.get()), SHADE_ALL, s->shade_cold),
+                                                         kBlock, 0));
         s->occ_trace = std::max(1, s->occ_trace);
         s->occ_shade = std::max(1, s->occ_shade);
         *out = s.release();
@@ -3170,7 +3192,7 @@ int luz_gpu_trace_paths(luz_gpu_scene* s, const LuzRenderParams* p, const int32_
                 CK(cudaMemsetAsync(s->ctrl, 0, sizeof(Ctrl), st));
                 k_raygen<<<(unsigned)((n + kBlock - 1) / kBlock), kBlock, 0, st>>>(w, s->pb, s->ctrl);
                 StageTimer T;
-                launch_bounces(s, w, st, launches, T, nullptr, s->pb, s->ctrl);
+                launch_bounces(s, w, st, launches, T, shade_mode(s), s->pb, s->ctrl);
                 k_path_color<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(w, s->pb);
                 CK(cudaMemcpyAsync(host.data(), s->pb.color, n * sizeof(float4), cudaMemcpyDeviceToHost, st));
                 finish_wave(s, st, nullptr, w.max_bounces);
@@ -3342,7 +3364,6 @@ int do_render_cached(luz_gpu_scene* s, luz_gpu_cache* c, const LuzRenderParams* 
     uint32_t* counts = D.get<uint32_t>(2, st);
     double* film = D.get<double>(3 * npix, st);
     float* d_out = D.get<float>(3 * npix, st);
-    const ShadeKernel shade_cached = shade_kernel(2);
     StageTimer T;
 
     WaveArgs w = base_args(s, p);
@@ -3388,7 +3409,7 @@ int do_render_cached(luz_gpu_scene* s, luz_gpu_cache* c, const LuzRenderParams* 
             CK(cudaMemsetAsync(tflag, 0, (std::size_t)w.n, st));
             CK(cudaMemsetAsync(c->loss, 0, sizeof(float), st));
             k_raygen<<<(unsigned)((w.n + kBlock - 1) / kBlock), kBlock, 0, st>>>(w, s->pb, s->ctrl);
-            launch_bounces(s, w, st, launches, T, shade_cached, s->pb, s->ctrl);
+            launch_bounces(s, w, st, launches, T, 2, s->pb, s->ctrl);
             k_cache_infer<<<(unsigned)(2 * s->sms), 128, kCacheInferSmem, st>>>(q, counts, 0, c->Wf, nullptr, s->pb.rad);
             k_cache_targets<<<(unsigned)((w.n + 255) / 256), 256, 0, st>>>(w, s->pb, rows, counts + 1);
             // about n / train_every rows: one step per batch of them (at most kCacheWaveSteps);

@@ -199,9 +199,10 @@ static __device__ LUZ_HIT_ATTR Hit make_hit_t(const DScene& S, const TRay& r, co
     return h;
 }
 
+template <bool COLD = true>
 __device__ __forceinline__ Hit make_hit(const DScene& S, const TRay& r, const THit& th)
 {
-    return S.k.cube_cross_spheres ? make_hit_t<true>(S, r, th) : make_hit_t<false>(S, r, th);
+    return COLD && S.k.cube_cross_spheres ? make_hit_t<true>(S, r, th) : make_hit_t<false>(S, r, th);
 }
 
 // ----------------------------------------------------------------------------- textures / colour
@@ -563,6 +564,7 @@ __device__ __forceinline__ F3 ray_dir_normalized(F3 d)   // Ray::_normalize (inc
 }
 
 // Material::evaluateBSDFCos / scatteringPDF for the BSDF-typed materials.
+template <bool COLD = true>
 static __device__ __noinline__ F3 bsdf_eval(const DScene& S, const GMaterial& m, const Hit& h, F3 ray_d, F3 dir)
 {
     const F3 view = safe_normalize(ray_d * -1.0f, h.n);
@@ -575,7 +577,8 @@ static __device__ __noinline__ F3 bsdf_eval(const DScene& S, const GMaterial& m,
         return ggx_dielectric_bsdfcos(color_at(S, m, h), h.n, view, dir, m.alpha, ei, et);
     }
     case MT_PRINCIPLED:
-        return principled_eval(S, m, h, ray_d, dir);
+        if constexpr (COLD) return principled_eval(S, m, h, ray_d, dir);
+        return F3{0.f, 0.f, 0.f};
     case MT_GLOSSY:   // Glossy::evaluateBSDFCos (Glossy.cpp:86-100): GGX lobe tinted by the colour, no Fresnel
         return ggx_reflection_bsdfcos(clamp_color01(color_at(S, m, h)), h.n, view, dir, m.alpha);
     case MT_DIFFUSE_GLOSSY: {   // DiffuseGlossy::evaluateBSDFCos (DiffuseGlossy.cpp:144-160)
@@ -588,6 +591,7 @@ static __device__ __noinline__ F3 bsdf_eval(const DScene& S, const GMaterial& m,
         return F3{0.f, 0.f, 0.f};
     }
 }
+template <bool COLD = true>
 static __device__ __noinline__ float bsdf_pdf(const DScene& S, const GMaterial& m, const Hit& h, F3 ray_d, F3 dir)
 {
     const F3 view = safe_normalize(ray_d * -1.0f, h.n);
@@ -599,7 +603,8 @@ static __device__ __noinline__ float bsdf_pdf(const DScene& S, const GMaterial& 
         return ggx_dielectric_pdf(h.n, view, dir, m.alpha, ei, et);
     }
     case MT_PRINCIPLED:
-        return principled_pdf(S, m, h, ray_d, dir);
+        if constexpr (COLD) return principled_pdf(S, m, h, ray_d, dir);
+        return 0.0f;
     case MT_GLOSSY:
         return ggx_reflection_pdf(h.n, view, dir, m.alpha);
     case MT_DIFFUSE_GLOSSY: {   // DiffuseGlossy::scatteringPDF (DiffuseGlossy.cpp:162-176)
@@ -629,10 +634,11 @@ __device__ __forceinline__ F3 ggx_reflection_sample(F3 d, F3 n, float alpha, con
     return dir;
 }
 
+template <bool COLD = true>
 __device__ __forceinline__ bool finish_bsdf(const DScene& S, const GMaterial& m, const Hit& h, F3 d, F3 dir, Scatter& sr)
 {
-    const float pdf = bsdf_pdf(S, m, h, d, dir);
-    const F3 bc = bsdf_eval(S, m, h, d, dir);
+    const float pdf = bsdf_pdf<COLD>(S, m, h, d, dir);
+    const F3 bc = bsdf_eval<COLD>(S, m, h, d, dir);
     if (pdf <= 0.0f || !isfinite(pdf) || maxc(bc) <= 0.0f) return false;
     sr.dir = dir;
     sr.spdf = pdf;
@@ -643,6 +649,7 @@ __device__ __forceinline__ bool finish_bsdf(const DScene& S, const GMaterial& m,
 }
 
 // Material::scatter for every type on the path; false = no scatter (emitter or failed sample).
+template <bool COLD = true>
 static __device__ __noinline__ bool scatter(const DScene& S, const GMaterial& m, const Hit& h, F3 d, const Key& k, Scatter& sr)
 {
     sr.specular = false;
@@ -676,7 +683,7 @@ static __device__ __noinline__ bool scatter(const DScene& S, const GMaterial& m,
             sr.specular = true;
             return true;
         }
-        return finish_bsdf(S, m, h, d, ggx_reflection_sample(d, h.n, m.alpha, k), sr);
+        return finish_bsdf<COLD>(S, m, h, d, ggx_reflection_sample(d, h.n, m.alpha, k), sr);
     }
     case MT_DIELECTRIC: {
         sr.absorb = (m.flags & MF_ABSORPTION) != 0;
@@ -708,17 +715,17 @@ static __device__ __noinline__ bool scatter(const DScene& S, const GMaterial& m,
         F3 dir;
         if (!can || sample1d(k, DIM_MATERIAL_DECISION) < (double)F) dir = reflect(d, hv);
         else dir = refr;
-        return finish_bsdf(S, m, h, d, dir, sr);
+        return finish_bsdf<COLD>(S, m, h, d, dir, sr);
     }
     case MT_GLOSSY:   // Glossy::scatter (Glossy.cpp:68-84)
-        return finish_bsdf(S, m, h, d, ggx_reflection_sample(d, h.n, m.alpha, k), sr);
+        return finish_bsdf<COLD>(S, m, h, d, ggx_reflection_sample(d, h.n, m.alpha, k), sr);
     case MT_DIFFUSE_GLOSSY: {   // DiffuseGlossy::scatter (DiffuseGlossy.cpp:118-142)
         F3 dir;
         if (sample1d(k, DIM_MATERIAL_DECISION) < (double)m.gweight) dir = ggx_reflection_sample(d, h.n, m.alpha, k);
         else dir = onb_local(make_onb(h.n), cosine_hemisphere(k, DIM_BSDF_DIRECTION));
-        return finish_bsdf(S, m, h, d, dir, sr);
+        return finish_bsdf<COLD>(S, m, h, d, dir, sr);
     }
-    case MT_PRINCIPLED: {
+    case MT_PRINCIPLED: if constexpr (COLD) {
         const F3 base = clamp_color01(color_at(S, m, h));
         sr.absorb = m.transmission > 0.0f && (m.flags & MF_ABSORPTION);
         sr.absorption = f3(m.absorption);
@@ -773,18 +780,20 @@ static __device__ __noinline__ bool scatter(const DScene& S, const GMaterial& m,
         } else {
             dir = ggx_reflection_sample(d, h.n, m.alpha, k);
         }
-        if (!finish_bsdf(S, m, h, d, dir, sr)) return false;
+        if (!finish_bsdf<COLD>(S, m, h, d, dir, sr)) return false;
         sr.subsurface = comp == 1;
         sr.thin = sr.subsurface && (m.flags & MF_THIN);
         sr.ss_radius_m = f3(m.ss_radius_m);
         return true;
     }
+        return false;
     default:
         return false;   // Emissive and BASIC do not scatter
     }
 }
 
 // scatterPDFValue (ColorHelper.cpp:38-86)
+template <bool COLD = true>
 static __device__ float scatter_pdf(const DScene& S, const Scatter& sr, const GMaterial& m, const Hit& h, F3 ray_d, F3 dir)
 {
     switch (sr.pdf) {
@@ -806,16 +815,17 @@ static __device__ float scatter_pdf(const DScene& S, const Scatter& sr, const GM
         return (1.0f - g2) / (4.0f * kPiF * den * sqrtf(den));
     }
     case PDF_BSDF:
-        return bsdf_pdf(S, m, h, ray_d, dir);
+        return bsdf_pdf<COLD>(S, m, h, ray_d, dir);
     default:
         return 0.0f;
     }
 }
 // scatterBSDFCos (ColorHelper.cpp:88-106)
+template <bool COLD = true>
 static __device__ F3 scatter_bsdfcos(const DScene& S, const Scatter& sr, const GMaterial& m, const Hit& h, F3 ray_d, F3 dir)
 {
-    if (sr.pdf == PDF_BSDF) return bsdf_eval(S, m, h, ray_d, dir);
-    return sr.att * scatter_pdf(S, sr, m, h, ray_d, dir);
+    if (sr.pdf == PDF_BSDF) return bsdf_eval<COLD>(S, m, h, ray_d, dir);
+    return sr.att * scatter_pdf<COLD>(S, sr, m, h, ray_d, dir);
 }
 // henyeyGreensteinDirection (ColorHelper.cpp:108-140)
 static __device__ __noinline__ F3 hg_direction(const Scatter& sr, const Key& k)
@@ -1260,6 +1270,7 @@ static __device__ int32_t mesh_pick(const DScene& S, const GMesh& M, const Key& 
     return S.index_pool[M.slot_offset + idx];
 }
 
+template <bool COLD = true>
 static __device__ __noinline__ bool light_surface_sample(const DScene& S, const GLight& L, F3 origin, const Key& k, LightSample& ls)
 {
     ls.valid = false;
@@ -1314,10 +1325,10 @@ static __device__ __noinline__ bool light_surface_sample(const DScene& S, const 
         ls.dir = dir;
         ls.pdf = 1.0f / sa;
         ls.tmax = root;
-        if (L.ies >= 0) ls.scale = ies_relative(S, L, dir * -1.0f);
+        if (COLD && L.ies >= 0) ls.scale = ies_relative(S, L, dir * -1.0f);
         return isfinite(ls.pdf) && ls.pdf > 0.0f && ls.tmax > kTMin;
     }
-    case LK_MESH: {
+    case LK_MESH: if constexpr (COLD) {
         const GMesh M = S.meshes[L.mesh];
         double selected;
         const int32_t slot = mesh_pick(S, M, k, selected);
@@ -1339,7 +1350,8 @@ static __device__ __noinline__ bool light_surface_sample(const DScene& S, const 
         ls.tmax = dist;
         return isfinite(pdf) && pdf > 0.0f;
     }
-    case LK_INSTANCE: {
+        return false;
+    case LK_INSTANCE: if constexpr (COLD) {
         const GObject O = S.objects[L.object];
         const GMesh M = S.meshes[L.mesh];
         if (L.area <= 0.0) return false;
@@ -1375,6 +1387,7 @@ static __device__ __noinline__ bool light_surface_sample(const DScene& S, const 
         ls.tmax = dist;
         return isfinite(ls.pdf) && ls.pdf > 0.0f && isfinite(ls.tmax) && ls.tmax > kTMin;
     }
+        return false;
     case LK_DIRECTIONAL: {
         const GObject O = S.objects[L.object];
         ls.dir = f3(O.f) * -1.0f;
@@ -1388,6 +1401,7 @@ static __device__ __noinline__ bool light_surface_sample(const DScene& S, const 
 }
 
 // Hittable::pdfValue of light L toward direction vec from origin.
+template <bool COLD = true>
 static __device__ __noinline__ float light_pdf_value(const DScene& S, const GLight& L, F3 origin, F3 vec)
 {
     VolSample vs{nullptr, 0.0, true};
@@ -1412,7 +1426,7 @@ static __device__ __noinline__ float light_pdf_value(const DScene& S, const GLig
         const float ctm = sqrtf(1.0f - rr2);
         return 1.0f / (2.0f * kPiF * (rr2 / (1.0f + ctm)));
     }
-    case LK_MESH: {
+    case LK_MESH: if constexpr (COLD) {
         const GMesh M = S.meshes[L.mesh];
         if (M.tri_count <= 0 || M.total_area <= 0.0) return 0.0f;
         const TRay r = make_ray(origin, ray_dir_normalized(vec));
@@ -1429,7 +1443,8 @@ static __device__ __noinline__ float light_pdf_value(const DScene& S, const GLig
         if (c <= 0.0f) return 0.0f;
         return (float)((double)d2 / ((double)c * M.total_area));
     }
-    case LK_INSTANCE: {
+        return 0.0f;
+    case LK_INSTANCE: if constexpr (COLD) {
         if (L.area <= 0.0) return 0.0f;
         const float vl = sqrtf(len2(vec));
         if (!isfinite(vl) || vl <= 0.0f) return 0.0f;
@@ -1462,16 +1477,18 @@ __device__ __forceinline__ float light_select_prob(const DScene& S, int32_t i)
     return (float)(w / S.k.light_total_weight);
 }
 // lightPDFValue (ColorHelper.cpp:233-257)
+template <bool COLD = true>
 static __device__ LUZ_LIGHT_ATTR float lights_pdf(const DScene& S, F3 origin, F3 dir)
 {
     const int32_t n = S.k.light_count;
     if (n <= 0) return 0.0f;
-    if (n == 1) return light_pdf_value(S, S.lights[0], origin, dir);
+    if (n == 1) return light_pdf_value<COLD>(S, S.lights[0], origin, dir);
     float sum = 0.0f;
-    for (int32_t i = 0; i < n; i++) sum += light_select_prob(S, i) * light_pdf_value(S, S.lights[i], origin, dir);
+    for (int32_t i = 0; i < n; i++) sum += light_select_prob(S, i) * light_pdf_value<COLD>(S, S.lights[i], origin, dir);
     return sum;
 }
 // selectLightIndex + sampleLight (ColorHelper.cpp:190-231, 925-971)
+template <bool COLD = true>
 static __device__ LUZ_LIGHT_ATTR bool sample_light(const DScene& S, F3 origin, const Key& k, LightSample& ls)
 {
     ls.valid = false;
@@ -1491,14 +1508,14 @@ static __device__ LUZ_LIGHT_ATTR bool sample_light(const DScene& S, F3 origin, c
     const GLight L = S.lights[idx];
     LightSample s;
     s.scale = 1.0f;
-    if (!light_surface_sample(S, L, origin, k, s)) return false;
+    if (!light_surface_sample<COLD>(S, L, origin, k, s)) return false;
     ls.dir = s.dir;
     ls.pdf = s.pdf * sel;
     ls.tmax = s.tmax;
     if (ls.pdf <= 0.0f || ls.tmax <= kTMin || !isfinite(ls.pdf) || !(ls.tmax == ls.tmax)) return false;
     if (!isfinite(ls.tmax) && L.kind != LK_DIRECTIONAL) return false;
     ls.emitted = f3(L.emitted);
-    if (L.ies >= 0) ls.emitted = ls.emitted * s.scale;
+    if (COLD && L.ies >= 0) ls.emitted = ls.emitted * s.scale;
     if (maxc(ls.emitted) <= 0.0f) return false;
     ls.light = idx;
     ls.valid = true;

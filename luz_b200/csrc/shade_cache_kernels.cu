@@ -9,7 +9,7 @@ namespace luz {
 
 ShadeKernel shade_kernel_cached()
 {
-    return k_shade<2>;
+    return k_shade<2, SHADE_ALL, true>;
 }
 
 }  // namespace luz

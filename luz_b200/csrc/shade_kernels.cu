@@ -22,19 +22,19 @@
 
 namespace luz {
 
-BatchShadeKernel batch_shade_kernel(int mode)
+BatchShadeKernel batch_shade_kernel(int mode, bool cold)
 {
-    return mode == 1 ? k_shade_batch<1> : k_shade_batch<0>;
+    return mode == 1 ? k_shade_batch<1, true> : cold ? k_shade_batch<0, true> : k_shade_batch<0, false>;
 }
 
-ShadeKernel shade_kernel(int mode)
+ShadeKernel shade_kernel(int mode, int part, bool cold)
 {
-    switch (mode) {
-    case 1: return k_shade<1>;
-    case 2: return shade_kernel_cached();
-    case 3: return k_shade<3>;
-    default: return k_shade<0>;
-    }
+    if (mode == 2) return shade_kernel_cached();
+    if (mode == 3) return cold ? k_shade<3, SHADE_ALL, true> : k_shade<3, SHADE_ALL, false>;
+    if (part == SHADE_MISSES) return cold ? k_shade_misses<0, true> : k_shade_misses<0, false>;
+    if (mode == 1) return part == SHADE_HITS ? k_shade<1, SHADE_HITS, true> : k_shade<1, SHADE_ALL, true>;
+    if (cold) return part == SHADE_HITS ? k_shade<0, SHADE_HITS, true> : k_shade<0, SHADE_ALL, true>;
+    return part == SHADE_HITS ? k_shade<0, SHADE_HITS, false> : k_shade<0, SHADE_ALL, false>;
 }
 
 }  // namespace luz

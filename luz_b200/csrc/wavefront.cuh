@@ -9,10 +9,6 @@ namespace luz {
 
 constexpr int kMaxBounceSlots = 256;
 constexpr int kBlock = 128;
-#ifndef LUZ_SHADE_BLOCK
-#define LUZ_SHADE_BLOCK 128
-#endif
-constexpr int kShadeBlock = LUZ_SHADE_BLOCK;   // threads per block of the shade kernels
 constexpr int kShadeClasses = 10;           // 0 = miss, 1..9 = material type of the hit
 
 struct Ctrl {
@@ -535,22 +531,32 @@ __device__ __forceinline__ void cache_inputs(const WaveArgs& w, const Hit& h, co
 }
 
 // MODE 0: plain; 1: with the caustic photon map; 2: radiance-cache render;
-// 3: adjoint (gradient) passes.
-template <int MODE>
+// 3: adjoint (gradient) passes. PART: the paths the kernel shades, SHADE_ALL of them, or
+// those that hit something or missed only (k_shade_hits, k_shade_misses).
+enum ShadePart : int { SHADE_ALL = 0, SHADE_HITS = 1, SHADE_MISSES = 2 };
+// COLD: the scene may hold what few scenes do (shade_cold); without it the kernel carries
+// neither that code nor the registers its calls take from the rest.
+template <int MODE, int PART, bool COLD>
 static __device__ void shade_path(const DScene& S, const WaveArgs& w, const PathBuf& P, uint32_t p, int bounce, ShadeOut& out)
 {
     out.cont = false;
     out.sh[0] = out.sh[1] = false;
     out.xobj = -1;
     out.xprim = -1;
-    const float4 t4 = P.thr[p], r4 = P.rad[p];
+    // A path starts with throughput 1, no radiance, nothing pending and a specular previous
+    // vertex: the first bounce knows that, and ray generation does not write it.
+    float4 t4 = make_float4(1.f, 1.f, 1.f, 0.f), r4 = make_float4(0.f, 0.f, 0.f, __uint_as_float(PF_PREV_SPECULAR));
+    if (bounce > 0) {
+        t4 = P.thr[p];
+        r4 = P.rad[p];
+    }
     F3 thr{t4.x, t4.y, t4.z};
     F3 rad{r4.x, r4.y, r4.z};
     uint32_t flags = __float_as_uint(r4.w);
     const float prev_pdf = t4.w;
     F3 pend_in{0.f, 0.f, 0.f};   // the previous vertex's light samples, as the shadow test left them
 
-    {
+    if (bounce > 0) {
         const float4 a = P.pend0[p], b = P.pend1[p];
         pend_in = F3{a.x, a.y, a.z} + F3{b.x, b.y, b.z};
         rad = (rad + F3{a.x, a.y, a.z}) + F3{b.x, b.y, b.z};
@@ -573,8 +579,8 @@ static __device__ void shade_path(const DScene& S, const WaveArgs& w, const Path
     F3 pend0{0.f, 0.f, 0.f}, pend1{0.f, 0.f, 0.f};
     const float4 ro = P.ray_o[p], rd = P.ray_d[p];
     const TRay ray = make_ray_x(F3{ro.x, ro.y, ro.z}, F3{rd.x, rd.y, rd.z}, __float_as_int(ro.w), __float_as_int(rd.w));
-    const float4 h4 = P.hit[p];
-    const int32_t obj = __float_as_int(h4.w);
+    const float4 h4 = PART == SHADE_MISSES ? make_float4(kInf, 0.f, 0.f, __int_as_float(-1)) : P.hit[p];
+    const int32_t obj = PART == SHADE_MISSES ? -1 : __float_as_int(h4.w);
     const uint32_t pix = P.pixel[p];
     const Key k = path_key(w, pix % (uint32_t)w.width, pix / (uint32_t)w.width, P.sample[p], (uint32_t)bounce);
     const bool prev_spec = (flags & PF_PREV_SPECULAR) != 0;
@@ -593,10 +599,10 @@ static __device__ void shade_path(const DScene& S, const WaveArgs& w, const Path
         }
     }
 
-    if (obj < 0) {   // miss (ColorHelper.cpp:1169-1210)
+    if (PART != SHADE_HITS && obj < 0) {   // miss (ColorHelper.cpp:1169-1210)
         float env_mis = 1.0f;
         const bool need_pdf = bounce > 0 && !prev_spec && (flags & PF_PREV_SVIL);
-        const bool need_rad = (S.k.sky == 3 || S.k.sky == 2) && S.k.env.present;
+        const bool need_rad = (S.k.sky == 3 || (COLD && S.k.sky == 2)) && S.k.env.present;
         F3 env_rad{0.f, 0.f, 0.f};
         float env_p = 0.0f;
         if ((need_pdf && S.k.env.lighting) || need_rad) env_query(S, ray.d, need_rad, need_pdf && S.k.env.lighting, env_rad, env_p);
@@ -608,9 +614,12 @@ static __device__ void shade_path(const DScene& S, const WaveArgs& w, const Path
         }
         F3 sky;
         if (S.k.sky == 1) {   // SKY_LINEAR: _calculateSkyInterpolation (Atmospherics.cpp:44-53), skyline 0.5
-            const float tl = 0.5f * ((ray.d.y / sqrtf(len2(ray.d))) + 1.0f);
+            // (rounded as every instantiation has it: left to the compiler, which product of the
+            // squared length is fused depends on what else the kernel holds)
+            const float l2 = __fmaf_rn(ray.d.z, ray.d.z, __fmaf_rn(ray.d.y, ray.d.y, __fmul_rn(ray.d.x, ray.d.x)));
+            const float tl = 0.5f * ((ray.d.y / sqrtf(l2)) + 1.0f);
             sky = (F3{1.0f, 1.0f, 1.0f} * (1.0f - tl)) + (F3{0.5f, 0.7f, 1.0f} * tl);
-        } else if (S.k.sky == 2) {   // sampleAtmosphereSky (ColorHelper.cpp:590-605)
+        } else if (COLD && S.k.sky == 2) {   // sampleAtmosphereSky (ColorHelper.cpp:590-605)
             double ao[3], ad[3];
             atmos_ray(w, P, p, bounce, ray, ao, ad);
             const AtmosSample a = atmos_segment(S, ao, ad, kDblMax);
@@ -628,27 +637,27 @@ static __device__ void shade_path(const DScene& S, const WaveArgs& w, const Path
         } else {
             sky = f3(S.k.background) * env_mis;
         }
-        if (bounce == 0 && w.nfor) store_miss_features(P, p, sky);   // env_mis is 1 at bounce 0
+        if (COLD && bounce == 0 && w.nfor) store_miss_features(P, p, sky);   // env_mis is 1 at bounce 0
         F3 contrib = thr * sky;
         if (bounce > 0 && S.k.has_constant_background_light) contrib = clamp_bg_miss(S, contrib);
         rad = rad + clamp_ray_color(contrib);
         goto done;
     }
-    {
+    if constexpr (PART != SHADE_MISSES) {
         THit th{h4.x, obj, P.hit_prim[p], h4.y, h4.z};
-        Hit h = make_hit(S, ray, th);
+        Hit h = make_hit<COLD>(S, ray, th);
         // The material is read where it lies (L1-cached global memory); only a Metal whose
         // roughness comes from a texture gets a resolved copy.
         const GMaterial* mp = S.materials + h.material;
         GMaterial m_res;
-        if (mp->rtexture >= 0) {
+        if (COLD && mp->rtexture >= 0) {
             m_res = *mp;
             resolve_material(S, m_res, h);
             mp = &m_res;
         }
         const GMaterial& m = *mp;
-        if (bounce == 0 && w.nfor) store_hit_features(S, P, p, h, m);
-        if (bounce == 0 && S.k.sky == 2) {   // compositePrimaryAtmosphereSegment (ColorHelper.cpp:645-659)
+        if (COLD && bounce == 0 && w.nfor) store_hit_features(S, P, p, h, m);
+        if (COLD && bounce == 0 && S.k.sky == 2) {   // compositePrimaryAtmosphereSegment (ColorHelper.cpp:645-659)
             double ao[3], ad[3];
             atmos_ray(w, P, p, bounce, ray, ao, ad);
             const AtmosSample a = atmos_segment(S, ao, ad, primary_atmos_tmax(S, ao, ad, (double)h.t));
@@ -658,9 +667,9 @@ static __device__ void shade_path(const DScene& S, const WaveArgs& w, const Path
         }
         const F3 emitted = m.type == MT_EMISSIVE ? f3(m.color) : F3{0.f, 0.f, 0.f};
         Scatter sr;
-        if (!scatter(S, m, h, ray.d, k, sr)) {
+        if (!scatter<COLD>(S, m, h, ray.d, k, sr)) {
             // previousScatterOrigin: read only after a non-specular scatter, whose hit point is this ray's origin
-            const float plp = (!prev_spec && S.k.light_count > 0) ? lights_pdf(S, ray.o, ray.d) : 0.0f;
+            const float plp = (!prev_spec && S.k.light_count > 0) ? lights_pdf<COLD>(S, ray.o, ray.d) : 0.0f;
             const float wgt = prev_spec ? 1.0f : power_heuristic(prev_pdf, plp);
             rad = rad + clamp_ray_color((thr * emitted) * wgt);
             if (MODE == 3 && w.adjoint && w.grad_emission && m.type == MT_EMISSIVE) {   // an emitter hit
@@ -672,7 +681,7 @@ static __device__ void shade_path(const DScene& S, const WaveArgs& w, const Path
             }
             goto done;
         }
-        relocate_subsurface(S, m, h, sr, ray.d, k);
+        if constexpr (COLD) relocate_subsurface(S, m, h, sr, ray.d, k);
         if (!h.volume) {
             out.xobj = h.obj;
             out.xprim = h.prim;
@@ -740,9 +749,9 @@ static __device__ void shade_path(const DScene& S, const WaveArgs& w, const Path
             bool go = true;
             if (prob < 1.0f && sample1d(k, DIM_LIGHT_STRATEGY) >= (double)prob) go = false;
             LightSample ls;
-            if (go && sample_light(S, h.p, k, ls) && leaves_opaque(m, h, ls.dir)) {
-                const float sp = scatter_pdf(S, sr, m, h, ray.d, ls.dir);
-                const F3 bc = scatter_bsdfcos(S, sr, m, h, ray.d, ls.dir);
+            if (go && sample_light<COLD>(S, h.p, k, ls) && leaves_opaque(m, h, ls.dir)) {
+                const float sp = scatter_pdf<COLD>(S, sr, m, h, ray.d, ls.dir);
+                const F3 bc = scatter_bsdfcos<COLD>(S, sr, m, h, ray.d, ls.dir);
                 if (!(sp <= 0.0f || !isfinite(sp) || maxc(bc) <= 0.0f)) {
                     const float mis = power_heuristic(ls.pdf, sp);
                     const F3 c = (bc * ls.emitted) * (mis / (ls.pdf * prob));
@@ -785,8 +794,8 @@ static __device__ void shade_path(const DScene& S, const WaveArgs& w, const Path
                 }
             }
             if (ls.valid && leaves_opaque(m, h, ls.dir)) {
-                const float sp = scatter_pdf(S, sr, m, h, ray.d, ls.dir);
-                const F3 bc = scatter_bsdfcos(S, sr, m, h, ray.d, ls.dir);
+                const float sp = scatter_pdf<COLD>(S, sr, m, h, ray.d, ls.dir);
+                const F3 bc = scatter_bsdfcos<COLD>(S, sr, m, h, ray.d, ls.dir);
                 if (!(sp <= 0.0f || !isfinite(sp) || maxc(bc) <= 0.0f)) {
                     const float mis = power_heuristic(ls.pdf, sp);
                     F3 c = (bc * ls.emitted) * (mis / (ls.pdf * prob));
@@ -822,7 +831,7 @@ static __device__ void shade_path(const DScene& S, const WaveArgs& w, const Path
         if (!leaves_opaque(m, h, dir)) goto done;
         // For a BSDF record this is scatteringPDF of the sampled direction with the same
         // inputs that produced sr.spdf, so the stored value is reused.
-        const float pdf = sr.pdf == PDF_BSDF ? sr.spdf : scatter_pdf(S, sr, m, h, ray.d, dir);
+        const float pdf = sr.pdf == PDF_BSDF ? sr.spdf : scatter_pdf<COLD>(S, sr, m, h, ray.d, dir);
         if (pdf <= 0.0f || !isfinite(pdf)) goto done;
         thr = clamp_ray_color(thr * att);
         if (terminated(thr) || !russian_roulette(thr, bounce, k)) goto done;
@@ -842,7 +851,7 @@ static __device__ void shade_path(const DScene& S, const WaveArgs& w, const Path
             w.adj_rough[p].dc[1] = dl.y;
             w.adj_rough[p].dc[2] = dl.z;
         }
-        const bool svil = ((S.k.sky == 3 || S.k.sky == 2) && S.k.env.lighting)
+        const bool svil = ((S.k.sky == 3 || (COLD && S.k.sky == 2)) && S.k.env.lighting)
                        || (S.k.has_constant_background_light && sr.pdf != PDF_BSDF);
         flags = (svil ? PF_PREV_SVIL : 0u) | (flags & PF_CACHE_DONE);
         P.thr[p] = make_float4(thr.x, thr.y, thr.z, pdf);
@@ -878,12 +887,12 @@ __device__ __forceinline__ F3 clean(F3 c)   // cleanColor (Threads.cpp:122-137)
 // Shade-stage kernels k_shade<mode> (shade_kernels.cu): 0 plain, 1 with the
 // caustic estimate, 2 radiance-cache render, 3 adjoint replay.
 using ShadeKernel = void (*)(const DScene*, WaveArgs, PathBuf, Ctrl*, int);
-ShadeKernel shade_kernel(int mode);
+ShadeKernel shade_kernel(int mode, int part, bool cold);
 ShadeKernel shade_kernel_cached();   // k_shade<2>, in its own translation unit
 
 // Multi-scene waves: every path finds its segment in P.seg, the segment's WaveArgs
 // in segs and its scene in scenes[segs[seg].batch_scene]. Modes 0 and 1 as above.
 using BatchShadeKernel = void (*)(const DScene*, const WaveArgs*, PathBuf, Ctrl*, int);
-BatchShadeKernel batch_shade_kernel(int mode);
+BatchShadeKernel batch_shade_kernel(int mode, bool cold);
 
 }  // namespace luz
