@@ -164,6 +164,21 @@ __global__ void k_cache_pack(const float* W, __half* Wf, __half* Wb)
     Wb[L.b + k * (L.N + 8) + n] = h;
 }
 
+// Records of n rows of inputs and targets (NULL: zeros).
+__global__ void k_cache_records(const float* in, const float* target, int n, CacheRecord* out)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    CacheRecord q;
+#pragma unroll
+    for (int f = 0; f < kCacheIn; f++) q.in[f] = in[(size_t)kCacheIn * i + f];
+#pragma unroll
+    for (int c = 0; c < 3; c++) q.v[c] = target ? target[3 * (size_t)i + c] : 0.0f;
+    q.path = 0;
+    q.pad[0] = q.pad[1] = 0.0f;
+    out[i] = q;
+}
+
 __device__ __forceinline__ void cache_load_smem(__half* dst, const __half* src, int halves)
 {
     const int4* s = reinterpret_cast<const int4*>(src);

@@ -972,6 +972,48 @@ template <class T> T* dupload(const std::vector<T>& v)
     return p;
 }
 
+// Device buffers of one call, from the device's scratch pool in the order of their stream,
+// given back to it on every exit path.
+struct DeviceScratch {
+    std::vector<std::pair<void*, cudaStream_t>> ptrs;
+    // n elements, not initialised
+    template <class T> T* raw(int64_t n, cudaStream_t st)
+    {
+        cudaError_t e = cudaSuccess;
+        const cudaMemPool_t pool = luz_scratch_pool(&e);
+        CK(e);
+        void* p = nullptr;
+        CK(cudaMallocFromPoolAsync(&p, sizeof(T) * (std::size_t)std::max<int64_t>(n, 1), pool, st));
+        ptrs.push_back({p, st});
+        return static_cast<T*>(p);
+    }
+    // n elements set to zero
+    template <class T> T* get(int64_t n, cudaStream_t st)
+    {
+        T* p = raw<T>(n, st);
+        CK(cudaMemsetAsync(p, 0, sizeof(T) * (std::size_t)std::max<int64_t>(n, 1), st));
+        return p;
+    }
+    ~DeviceScratch()
+    {
+        for (auto& p : ptrs) cudaFreeAsync(p.first, p.second);
+    }
+};
+
+// Handles (scenes, caches) alive per device: the last one's end empties the scratch pool.
+std::mutex g_handles_mu;
+std::map<int, int> g_handles;
+void handle_opened(int device)
+{
+    std::lock_guard<std::mutex> lock(g_handles_mu);
+    g_handles[device]++;
+}
+void handle_closed(int device)
+{
+    std::lock_guard<std::mutex> lock(g_handles_mu);
+    if (--g_handles[device] == 0) luz_scratch_trim(device);
+}
+
 uint64_t next_scene_uid()
 {
     static std::atomic<uint64_t> n{0};
@@ -991,10 +1033,46 @@ int guard(const std::function<int()>& f)
     }
 }
 
+std::mutex g_scratch_mu;
+std::vector<cudaMemPool_t> g_scratch;   // per device, created on first use, kept for the process
+
 }  // namespace
+
+cudaMemPool_t luz_scratch_pool(cudaError_t* err)
+{
+    int device = 0;
+    *err = cudaGetDevice(&device);
+    if (*err != cudaSuccess) return nullptr;
+    std::lock_guard<std::mutex> lock(g_scratch_mu);
+    if ((int)g_scratch.size() <= device) g_scratch.resize(device + 1, nullptr);
+    if (!g_scratch[device]) {
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = device;
+        cudaMemPool_t pool = nullptr;
+        *err = cudaMemPoolCreate(&pool, &props);
+        if (*err != cudaSuccess) return nullptr;
+        unsigned long long keep = kScratchKeep;
+        *err = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        if (*err != cudaSuccess) {
+            cudaMemPoolDestroy(pool);
+            return nullptr;
+        }
+        g_scratch[device] = pool;
+    }
+    return g_scratch[device];
+}
+
+void luz_scratch_trim(int device)
+{
+    std::lock_guard<std::mutex> lock(g_scratch_mu);
+    if (device >= 0 && device < (int)g_scratch.size() && g_scratch[device]) cudaMemPoolTrimTo(g_scratch[device], 0);
+}
 
 struct luz_gpu_scene {
     int device = 0;
+    bool counted = false;            // among the device's live handles
     std::unique_ptr<ScenePack> pack;
     DScene ds{};
     DScene* dds = nullptr;           // device copy of ds: k_shade reads it through a pointer so that
@@ -1131,6 +1209,7 @@ struct luz_gpu_scene {
             } catch (const Status& e) {
                 free_paths();
                 (void)cudaGetLastError();   // clears the allocation error
+                luz_scratch_trim(device);
                 if (e.code != LUZ_E_CUDA || n <= floor_n) throw;
                 n = std::max(floor_n, n / 2);
             }
@@ -1157,6 +1236,7 @@ struct luz_gpu_scene {
         for (cudaEvent_t e : {lane_setup, lane_done, lane_acc[0], lane_acc[1]})
             if (e) cudaEventDestroy(e);
         if (stream2) cudaStreamDestroy(stream2);
+        if (counted) handle_closed(device);
     }
     void ensure_lanes()
     {
@@ -1672,22 +1752,6 @@ int do_render(luz_gpu_scene* s, const LuzRenderParams* p, float* d_out, cudaStre
     }
     return LUZ_OK;
 }
-
-// Device buffers of one luz_gpu_render_ex call, freed on every exit path.
-struct DeviceScratch {
-    std::vector<void*> ptrs;
-    template <class T> T* get(int64_t n, cudaStream_t st)
-    {
-        T* p = dalloc<T>((std::size_t)n);
-        ptrs.push_back(p);
-        CK(cudaMemsetAsync(p, 0, sizeof(T) * (std::size_t)std::max<int64_t>(n, 1), st));
-        return p;
-    }
-    ~DeviceScratch()
-    {
-        for (void* p : ptrs) cudaFree(p);
-    }
-};
 
 // Scene::setAdaptive* validation (src/scene/Scene.cpp:193-222).
 void check_adaptive(const LuzAdaptiveParams* a)
@@ -2776,6 +2840,8 @@ int luz_gpu_scene_create(const LuzSceneDesc* desc, int32_t device, luz_gpu_scene
         s->pack.reset(pack_scene(desc));
         s->device = device;
         CK(cudaSetDevice(device));
+        handle_opened(device);
+        s->counted = true;
         CK(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking));
         CK(cudaEventCreate(&s->ev0));
         CK(cudaEventCreate(&s->ev1));
@@ -3170,47 +3236,38 @@ int luz_gpu_trace_paths(luz_gpu_scene* s, const LuzRenderParams* p, const int32_
         clear_error(s, st);
         prepare_caustics(s, p, st);
         const int64_t chunk = s->reserve_paths(std::min<int64_t>(count, kWaveTarget));
-        int32_t* dx = dalloc<int32_t>(chunk);
-        int32_t* dy = dalloc<int32_t>(chunk);
-        int32_t* dsm = dalloc<int32_t>(chunk);
+        DeviceScratch D;
+        int32_t* dx = D.raw<int32_t>(chunk, st);
+        int32_t* dy = D.raw<int32_t>(chunk, st);
+        int32_t* dsm = D.raw<int32_t>(chunk, st);
         std::vector<float4> host((std::size_t)chunk);
         int64_t launches = 0;
-        try {
-            WaveArgs w = base_args(s, p);
-            for (int64_t b = 0; b < count; b += chunk) {
-                const int64_t n = std::min(chunk, count - b);
-                CK(cudaMemcpyAsync(dx, x + b, n * 4, cudaMemcpyHostToDevice, st));
-                CK(cudaMemcpyAsync(dy, y + b, n * 4, cudaMemcpyHostToDevice, st));
-                CK(cudaMemcpyAsync(dsm, sample + b, n * 4, cudaMemcpyHostToDevice, st));
-                w.list_mode = 1;
-                w.list_x = dx;
-                w.list_y = dy;
-                w.list_s = dsm;
-                w.n = n;
-                w.s_count = 1;
-                w.pix_count = (int32_t)n;
-                CK(cudaMemsetAsync(s->ctrl, 0, sizeof(Ctrl), st));
-                k_raygen<<<(unsigned)((n + kBlock - 1) / kBlock), kBlock, 0, st>>>(w, s->pb, s->ctrl);
-                StageTimer T;
-                launch_bounces(s, w, st, launches, T, shade_mode(s), s->pb, s->ctrl);
-                k_path_color<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(w, s->pb);
-                CK(cudaMemcpyAsync(host.data(), s->pb.color, n * sizeof(float4), cudaMemcpyDeviceToHost, st));
-                finish_wave(s, st, nullptr, w.max_bounces);
-                for (int64_t i = 0; i < n; i++) {
-                    rgb_out[3 * (b + i)] = host[i].x;
-                    rgb_out[3 * (b + i) + 1] = host[i].y;
-                    rgb_out[3 * (b + i) + 2] = host[i].z;
-                }
+        WaveArgs w = base_args(s, p);
+        for (int64_t b = 0; b < count; b += chunk) {
+            const int64_t n = std::min(chunk, count - b);
+            CK(cudaMemcpyAsync(dx, x + b, n * 4, cudaMemcpyHostToDevice, st));
+            CK(cudaMemcpyAsync(dy, y + b, n * 4, cudaMemcpyHostToDevice, st));
+            CK(cudaMemcpyAsync(dsm, sample + b, n * 4, cudaMemcpyHostToDevice, st));
+            w.list_mode = 1;
+            w.list_x = dx;
+            w.list_y = dy;
+            w.list_s = dsm;
+            w.n = n;
+            w.s_count = 1;
+            w.pix_count = (int32_t)n;
+            CK(cudaMemsetAsync(s->ctrl, 0, sizeof(Ctrl), st));
+            k_raygen<<<(unsigned)((n + kBlock - 1) / kBlock), kBlock, 0, st>>>(w, s->pb, s->ctrl);
+            StageTimer T;
+            launch_bounces(s, w, st, launches, T, shade_mode(s), s->pb, s->ctrl);
+            k_path_color<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(w, s->pb);
+            CK(cudaMemcpyAsync(host.data(), s->pb.color, n * sizeof(float4), cudaMemcpyDeviceToHost, st));
+            finish_wave(s, st, nullptr, w.max_bounces);
+            for (int64_t i = 0; i < n; i++) {
+                rgb_out[3 * (b + i)] = host[i].x;
+                rgb_out[3 * (b + i) + 1] = host[i].y;
+                rgb_out[3 * (b + i) + 2] = host[i].z;
             }
-        } catch (...) {
-            cudaFree(dx);
-            cudaFree(dy);
-            cudaFree(dsm);
-            throw;
         }
-        cudaFree(dx);
-        cudaFree(dy);
-        cudaFree(dsm);
         return LUZ_OK;
     });
 }
@@ -3223,27 +3280,18 @@ int luz_gpu_trace_rays(luz_gpu_scene* s, const float* rays, int64_t count, int32
         if (count <= 0) return LUZ_OK;
         CK(cudaSetDevice(s->device));
         cudaStream_t st = s->stream;
-        float* dr = dalloc<float>((std::size_t)(8 * count));
-        LuzHit* dh = dalloc<LuzHit>((std::size_t)count);
-        int32_t* dk = volume_key ? dalloc<int32_t>((std::size_t)(4 * count)) : nullptr;
-        try {
-            clear_error(s, st);
-            CK(cudaMemcpyAsync(dr, rays, sizeof(float) * 8 * count, cudaMemcpyHostToDevice, st));
-            if (dk) CK(cudaMemcpyAsync(dk, volume_key, sizeof(int32_t) * 4 * count, cudaMemcpyHostToDevice, st));
-            kTraceRayKernels[s->ds.k.features & TF_ALL]<<<(unsigned)((count + 127) / 128), 128, 0, st>>>(
-                s->ds, dr, count, any_hit, seed, dk, dh);
-            CK(cudaGetLastError());
-            CK(cudaMemcpyAsync(out, dh, sizeof(LuzHit) * count, cudaMemcpyDeviceToHost, st));
-            finish_status(s, st);
-        } catch (...) {
-            cudaFree(dr);
-            cudaFree(dh);
-            if (dk) cudaFree(dk);
-            throw;
-        }
-        cudaFree(dr);
-        cudaFree(dh);
-        if (dk) cudaFree(dk);
+        DeviceScratch D;
+        float* dr = D.raw<float>(8 * count, st);
+        LuzHit* dh = D.raw<LuzHit>(count, st);
+        int32_t* dk = volume_key ? D.raw<int32_t>(4 * count, st) : nullptr;
+        clear_error(s, st);
+        CK(cudaMemcpyAsync(dr, rays, sizeof(float) * 8 * count, cudaMemcpyHostToDevice, st));
+        if (dk) CK(cudaMemcpyAsync(dk, volume_key, sizeof(int32_t) * 4 * count, cudaMemcpyHostToDevice, st));
+        kTraceRayKernels[s->ds.k.features & TF_ALL]<<<(unsigned)((count + 127) / 128), 128, 0, st>>>(
+            s->ds, dr, count, any_hit, seed, dk, dh);
+        CK(cudaGetLastError());
+        CK(cudaMemcpyAsync(out, dh, sizeof(LuzHit) * count, cudaMemcpyDeviceToHost, st));
+        finish_status(s, st);
         return LUZ_OK;
     });
 }
@@ -3254,6 +3302,7 @@ int luz_gpu_trace_rays(luz_gpu_scene* s, const float* rays, int64_t count, int32
 
 struct luz_gpu_cache {
     int device = 0;
+    bool counted = false;
     LuzCacheParams prm{};
     float *W = nullptr, *G = nullptr, *m = nullptr, *v = nullptr, *loss = nullptr;
     __half *Wf = nullptr, *Wb = nullptr;
@@ -3263,6 +3312,7 @@ struct luz_gpu_cache {
         cudaSetDevice(device);
         for (void* p : {(void*)W, (void*)G, (void*)m, (void*)v, (void*)loss, (void*)Wf, (void*)Wb})
             if (p) cudaFree(p);
+        if (counted) handle_closed(device);
     }
 };
 
@@ -3320,16 +3370,19 @@ void cache_step(luz_gpu_cache* c, const CacheRecord* rows, const uint32_t* count
     cache_pack(c, st);
 }
 
-std::vector<CacheRecord> cache_rows(const float* inputs, const float* targets, int64_t n)
+// Device records of host rows (targets may be NULL), on the default stream.
+CacheRecord* cache_rows(DeviceScratch& D, const float* inputs, const float* targets, int64_t n)
 {
-    std::vector<CacheRecord> r((std::size_t)n);
-    for (int64_t i = 0; i < n; i++) {
-        CacheRecord& q = r[(std::size_t)i];
-        std::memset(&q, 0, sizeof(q));
-        for (int f = 0; f < kCacheIn; f++) q.in[f] = inputs[kCacheIn * i + f];
-        if (targets)
-            for (int k = 0; k < 3; k++) q.v[k] = targets[3 * i + k];
+    float* in = D.raw<float>(kCacheIn * n, 0);
+    CK(cudaMemcpyAsync(in, inputs, sizeof(float) * (std::size_t)(kCacheIn * n), cudaMemcpyHostToDevice, 0));
+    float* t = nullptr;
+    if (targets) {
+        t = D.raw<float>(3 * n, 0);
+        CK(cudaMemcpyAsync(t, targets, sizeof(float) * (std::size_t)(3 * n), cudaMemcpyHostToDevice, 0));
     }
+    CacheRecord* r = D.raw<CacheRecord>(n, 0);
+    k_cache_records<<<(unsigned)((n + 127) / 128), 128>>>(in, t, (int)n, r);
+    CK(cudaGetLastError());
     return r;
 }
 
@@ -3469,6 +3522,8 @@ int luz_gpu_cache_create(int32_t device, const LuzCacheParams* prm, luz_gpu_cach
         CK(cudaSetDevice(device));
         std::unique_ptr<luz_gpu_cache> c(new luz_gpu_cache);
         c->device = device;
+        handle_opened(device);
+        c->counted = true;
         c->prm = *prm;
         c->W = dalloc<float>(kCacheParams);
         c->G = dalloc<float>(kCacheParams);
@@ -3512,23 +3567,14 @@ int luz_gpu_cache_predict(luz_gpu_cache* c, const float* inputs, int64_t n, floa
         if (!rgb_out && n > 0) throw Status(LUZ_E_INVALID, "NULL argument.");
         if (n == 0) return LUZ_OK;
         CK(cudaSetDevice(c->device));
-        const std::vector<CacheRecord> r = cache_rows(inputs, nullptr, n);
-        CacheRecord* d = dupload(r);
-        float* o = nullptr;
-        try {
-            o = dalloc<float>((std::size_t)(3 * n));
-            const int tiles = (int)((n + 15) / 16);
-            k_cache_infer<<<(unsigned)std::max(1, std::min(tiles / 4 + 1, 1184)), 128, kCacheInferSmem>>>(
-                d, nullptr, (int)n, c->Wf, o, nullptr);
-            CK(cudaGetLastError());
-            CK(cudaMemcpy(rgb_out, o, sizeof(float) * 3 * (std::size_t)n, cudaMemcpyDeviceToHost));
-        } catch (...) {
-            cudaFree(d);
-            if (o) cudaFree(o);
-            throw;
-        }
-        cudaFree(d);
-        cudaFree(o);
+        DeviceScratch D;
+        const CacheRecord* d = cache_rows(D, inputs, nullptr, n);
+        float* o = D.raw<float>(3 * n, 0);
+        const int tiles = (int)((n + 15) / 16);
+        k_cache_infer<<<(unsigned)std::max(1, std::min(tiles / 4 + 1, 1184)), 128, kCacheInferSmem>>>(
+            d, nullptr, (int)n, c->Wf, o, nullptr);
+        CK(cudaGetLastError());
+        CK(cudaMemcpy(rgb_out, o, sizeof(float) * 3 * (std::size_t)n, cudaMemcpyDeviceToHost));
         return LUZ_OK;
     });
 }
@@ -3540,27 +3586,21 @@ int luz_gpu_cache_gradient(luz_gpu_cache* c, const float* inputs, const float* t
         cache_check_rows(c, inputs, n);
         if (!targets || n <= 0) throw Status(LUZ_E_INVALID, "Gradient needs rows and targets.");
         CK(cudaSetDevice(c->device));
-        const std::vector<CacheRecord> r = cache_rows(inputs, targets, n);
-        CacheRecord* d = dupload(r);
-        try {
-            CK(cudaMemset(c->G, 0, sizeof(float) * kCacheParams));
-            CK(cudaMemset(c->loss, 0, sizeof(float)));
-            k_cache_grad<<<(unsigned)((n + kCacheRowsPerBlock - 1) / kCacheRowsPerBlock), kCacheGradThreads, kCacheGradSmem>>>(
-                d, nullptr, 0, (int)n, c->Wf, c->Wb, c->G, c->loss);
-            CK(cudaGetLastError());
-            std::vector<float> g(kCacheParams);
-            float l = 0.f;
-            CK(cudaMemcpy(g.data(), c->G, sizeof(float) * kCacheParams, cudaMemcpyDeviceToHost));
-            CK(cudaMemcpy(&l, c->loss, sizeof(float), cudaMemcpyDeviceToHost));
-            CK(cudaMemset(c->G, 0, sizeof(float) * kCacheParams));
-            if (grad_out)
-                for (int i = 0; i < kCacheParams; i++) grad_out[i] = g[(std::size_t)i] / (kCacheLossScale * (float)n);
-            if (loss_out) *loss_out = (double)l / (double)n;
-        } catch (...) {
-            cudaFree(d);
-            throw;
-        }
-        cudaFree(d);
+        DeviceScratch D;
+        const CacheRecord* d = cache_rows(D, inputs, targets, n);
+        CK(cudaMemsetAsync(c->G, 0, sizeof(float) * kCacheParams, 0));
+        CK(cudaMemsetAsync(c->loss, 0, sizeof(float), 0));
+        k_cache_grad<<<(unsigned)((n + kCacheRowsPerBlock - 1) / kCacheRowsPerBlock), kCacheGradThreads, kCacheGradSmem>>>(
+            d, nullptr, 0, (int)n, c->Wf, c->Wb, c->G, c->loss);
+        CK(cudaGetLastError());
+        std::vector<float> g(kCacheParams);
+        float l = 0.f;
+        CK(cudaMemcpy(g.data(), c->G, sizeof(float) * kCacheParams, cudaMemcpyDeviceToHost));
+        CK(cudaMemsetAsync(c->G, 0, sizeof(float) * kCacheParams, 0));
+        CK(cudaMemcpy(&l, c->loss, sizeof(float), cudaMemcpyDeviceToHost));   // and the clear before it is done
+        if (grad_out)
+            for (int i = 0; i < kCacheParams; i++) grad_out[i] = g[(std::size_t)i] / (kCacheLossScale * (float)n);
+        if (loss_out) *loss_out = (double)l / (double)n;
         return LUZ_OK;
     });
 }
@@ -3574,22 +3614,16 @@ int luz_gpu_cache_train(luz_gpu_cache* c, const float* inputs, const float* targ
         if (n > c->prm.batch) throw Status(LUZ_E_INVALID, "More rows than the cache batch.");
         if (steps < 0) throw Status(LUZ_E_INVALID, "Step count must be non-negative.");
         CK(cudaSetDevice(c->device));
-        const std::vector<CacheRecord> r = cache_rows(inputs, targets, n);
-        CacheRecord* d = dupload(r);
-        try {
-            for (int i = 0; i < steps; i++) {
-                CK(cudaMemset(c->loss, 0, sizeof(float)));
-                cache_step(c, d, nullptr, 0, (int)n, 0);
-                CK(cudaGetLastError());
-                float l = 0.f;
-                CK(cudaMemcpy(&l, c->loss, sizeof(float), cudaMemcpyDeviceToHost));
-                if (loss_out) loss_out[i] = (double)l / (double)n;
-            }
-        } catch (...) {
-            cudaFree(d);
-            throw;
+        DeviceScratch D;
+        const CacheRecord* d = cache_rows(D, inputs, targets, n);
+        for (int i = 0; i < steps; i++) {
+            CK(cudaMemsetAsync(c->loss, 0, sizeof(float), 0));
+            cache_step(c, d, nullptr, 0, (int)n, 0);
+            CK(cudaGetLastError());
+            float l = 0.f;
+            CK(cudaMemcpy(&l, c->loss, sizeof(float), cudaMemcpyDeviceToHost));
+            if (loss_out) loss_out[i] = (double)l / (double)n;
         }
-        cudaFree(d);
         return LUZ_OK;
     });
 }

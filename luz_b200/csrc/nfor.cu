@@ -442,18 +442,24 @@ struct NforError {
         if (e_ != cudaSuccess) throw NforError{LUZ_E_CUDA, std::string(#x) + ": " + cudaGetErrorString(e_)}; \
     } while (0)
 
+// Scratch arrays of one call, from the device's pool, in the order of stream st.
 struct Buffers {
+    cudaStream_t st;
     std::vector<void*> p;
+    explicit Buffers(cudaStream_t s) : st(s) {}
     double* get(size_t n)
     {
+        cudaError_t e = cudaSuccess;
+        const cudaMemPool_t pool = luz_scratch_pool(&e);
+        NCK(e);
         void* q = nullptr;
-        NCK(cudaMalloc(&q, sizeof(double) * (n ? n : 1)));
+        NCK(cudaMallocFromPoolAsync(&q, sizeof(double) * (n ? n : 1), pool, st));
         p.push_back(q);
         return static_cast<double*>(q);
     }
     ~Buffers()
     {
-        for (void* q : p) cudaFree(q);
+        for (void* q : p) cudaFreeAsync(q, st);
     }
 };
 
@@ -471,7 +477,7 @@ void run_device(const double* ca, const double* cb, const double* cv, const doub
                 cudaStream_t st)
 {
     const size_t n = (size_t)width * height;
-    Buffers B;
+    Buffers B(st);
     const Img I{width, height};
     const dim3 blk(64), grd((unsigned)((width + 63) / 64), (unsigned)height);
     // firefly suppression of A, B and of their average (applyNFOR :989-996)
@@ -520,7 +526,6 @@ void run_device(const double* ca, const double* cb, const double* cv, const doub
     k_patch_dist<<<dgrid, 256, 0, st>>>(C, dist);
     k_regression_warp<<<rgrid_single, 128, 0, st>>>(C);
     NCK(cudaGetLastError());
-    NCK(cudaStreamSynchronize(st));   // the scratch buffers are freed on return
 }
 
 int do_nfor(int32_t device, const LuzNforBuffers* in, int32_t width, int32_t height, const LuzNforSettings* st,
@@ -534,7 +539,7 @@ int do_nfor(int32_t device, const LuzNforBuffers* in, int32_t width, int32_t hei
         throw NforError{LUZ_E_INVALID, "NFOR needs every buffer."};
     NCK(cudaSetDevice(device));
     const size_t n = (size_t)width * height;
-    Buffers B;
+    Buffers B(0);
     double* ca = B.get(3 * n);
     double* cb = B.get(3 * n);
     double* cv = B.get(n);

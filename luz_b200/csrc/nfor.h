@@ -1,5 +1,7 @@
 // NFOR denoiser entry shared by the render path (integrator.cu) and nfor.cu.
 #pragma once
+#include <cuda_runtime.h>
+
 
 #include <cstdint>
 #include <string>
@@ -8,9 +10,23 @@
 
 // Denoise::applyNFOR (src/core/Denoise/NFOR.cpp:977-1102) on device-resident
 // NFOR buffers laid out as LuzNforBuffers; writes width*height*3 doubles to
-// d_out on `stream` and synchronizes it. settings NULL = NFORSettings defaults.
+// d_out in `stream`'s order. settings NULL = NFORSettings defaults.
 // Returns LUZ_OK, or a LUZ_E_* code with its message in msg.
 int luz_nfor_on_device(const double* color_a, const double* color_b, const double* color_variance,
                        const double* features_a, const double* features_b, const double* feature_variance,
                        int32_t width, int32_t height, const LuzNforSettings* settings, double* d_out, void* stream,
                        std::string& msg);
+
+// Device scratch of single calls (ray batches, NFOR and adaptive buffers, gradients, cache
+// rows) comes from one stream-ordered pool per device instead of cudaMalloc: an allocation
+// and its release cost 0.6 ms there, and these calls make 3 to 45 of them. The pool keeps at
+// most kScratchKeep bytes between calls (what lies above goes back to the device at the next
+// synchronisation), gives all of it back when the last handle of the device is destroyed or
+// an allocation outside it fails, and orders reuse between streams and threads by the
+// streams' own dependencies.
+constexpr unsigned long long kScratchKeep = 2ull << 30;
+
+// The current device's scratch pool; on failure NULL, with the CUDA error in *err.
+cudaMemPool_t luz_scratch_pool(cudaError_t* err);
+// Gives what the pool of `device` holds unused back to the device.
+void luz_scratch_trim(int device);

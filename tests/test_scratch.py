@@ -1,0 +1,74 @@
+"""The scratch pool of single calls (ray batches, NFOR buffers, gradients, cache rows): calls
+from several threads share it without changing a result, and the memory it keeps goes back to
+the device with the last handle."""
+import subprocess
+import sys
+import threading
+
+import numpy as np
+import pytest
+
+from luz_b200 import native, scenes
+
+pytestmark = pytest.mark.gpu
+
+
+def buffers(w: int, h: int, seed: int) -> dict:
+    rng = np.random.default_rng(seed)
+    f = rng.random((h, w, 11))
+    return {"color_a": rng.random((h, w, 3)), "color_b": rng.random((h, w, 3)),
+            "color_variance": 0.01 + 0.1 * rng.random((h, w)), "features_a": f,
+            "features_b": f + 0.02 * rng.normal(size=f.shape), "feature_variance": np.full(f.shape, 2e-4)}
+
+
+def test_threads_share_the_pool():
+    w = scenes.mesh_glossy(32, 32, 1, 2, level=3)
+    handles = [native.GpuScene(w.scene.build()) for _ in range(2)]
+    rng = np.random.default_rng(3)
+    rays = np.zeros((5003, 8), np.float32)
+    rays[:, 0:3], rays[:, 3], rays[:, 7] = (0.0, 0.0, 4.0), 1e-3, np.inf
+    d = rng.normal(size=(5003, 3)) * 0.3 + (0.0, 0.0, -1.0)
+    rays[:, 4:7] = d / np.linalg.norm(d, axis=1, keepdims=True)
+    jobs = [lambda i=i: native.nfor_denoise(buffers(17 + 31 * i, 9 + 20 * i, i)) for i in range(4)]
+    jobs += [lambda g=g: g.trace_rays(rays).tobytes() for g in handles]
+    want = [j() for j in jobs]
+    got = [[] for _ in jobs]
+
+    def work(k):
+        for _ in range(5):
+            got[k].append(jobs[k]())
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(len(jobs))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for k, results in enumerate(got):
+        assert len(results) == 5
+        assert all(r == want[k] if isinstance(r, bytes) else np.array_equal(r, want[k]) for r in results), k
+    for g in handles:
+        g.close()
+
+
+def test_the_last_handle_gives_the_memory_back():
+    """In a process of its own: a 960x540 denoise leaves at most 2 GiB in the pool, and the
+    end of the last handle leaves what an idle process held before it (to 64 MiB)."""
+    code = """
+import numpy as np, torch
+from luz_b200 import native, scenes
+import sys; sys.path.insert(0, 'tests')
+from test_scratch import buffers
+torch.cuda.init(); torch.zeros(1, device='cuda')
+w = scenes.mesh_glossy(8, 8, 1, 1, level=2)
+g = native.GpuScene(w.scene.build()); native.nfor_denoise(buffers(8, 8, 1)); g.close()
+free0 = torch.cuda.mem_get_info()[0]
+g = native.GpuScene(w.scene.build())
+native.nfor_denoise(buffers(960, 540, 2))
+held = free0 - torch.cuda.mem_get_info()[0]
+g.close()
+left = free0 - torch.cuda.mem_get_info()[0]
+print(held >> 20, left >> 20)
+assert (64 << 20) < held <= (2 << 30) + (64 << 20) and left <= (64 << 20), (held, left)
+"""
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
