@@ -250,20 +250,32 @@ __global__ void k_patch_dist(RegArgs A, double* D)
 // time with one neighbour per lane, and reach the other lanes by shuffle.
 // Pair mode (bw2 >= 0): one pixel per warp, half 0 with bw1, half 1 with bw2.
 // Single mode: two pixels per warp, both with bw1.
-__global__ void __launch_bounds__(128) k_regression_warp(RegArgs A)
+// With a list (of *list_n entries, pixel << 1 | bandwidth) each half-warp takes entries of it.
+__device__ void regression_half(const RegArgs& A, long long pix, bool second);
+__global__ void __launch_bounds__(128) k_regression_warp(RegArgs A, const unsigned* list, const unsigned* list_n)
+{
+    const unsigned half = (threadIdx.x & 31u) >> 4;
+    const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const long long npix = (long long)A.I.w * A.I.h;
+    const bool pair = A.bw2 >= 0.0;
+    if (list) {
+        const long long n = *list_n, halves = 2ll * ((gridDim.x * blockDim.x) >> 5);
+        for (long long i = 2 * warp + half; i < n; i += halves) regression_half(A, list[i] >> 1, list[i] & 1u);
+        return;
+    }
+    const long long pix = pair ? warp : 2 * warp + half;
+    if (pix < npix) regression_half(A, pix, pair && half);   // the last odd pixel's half leaves alone
+}
+__device__ void regression_half(const RegArgs& A, long long pix, bool second)
 {
     const Img I = A.I;
     const unsigned lane = threadIdx.x & 31u, half = lane >> 4, j = lane & 15u;
     const unsigned hmask = half ? 0xffff0000u : 0x0000ffffu;
-    const bool pair = A.bw2 >= 0.0;
-    const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const long long pix = pair ? warp : 2 * warp + half;
     const long long npix = (long long)I.w * I.h;
-    if (pix >= npix) return;   // both halves of a warp leave together except the last odd pixel's half
     const int x = (int)(pix % I.w), y = (int)(pix / I.w);
     const int center = y * I.w + x;
-    const double bw = (pair && half) ? A.bw2 : A.bw1;
-    double* out = (pair && half) ? A.out2 : A.out1;
+    const double bw = second ? A.bw2 : A.bw1;
+    double* out = second ? A.out2 : A.out1;
     double M[kR];
 #pragma unroll
     for (int r = 0; r < kR; r++) M[r] = (j < (unsigned)kR && r == (int)j) ? 1e-4 : 0.0;   // ridge on the diagonal
@@ -347,6 +359,121 @@ __global__ void __launch_bounds__(128) k_regression_warp(RegArgs A)
         if (j >= (unsigned)kR && j < (unsigned)kR + 3) out[3 * center + (j - kR)] = M[0];
     } else if (j == 0) {
         fallback(I, A.image, A.var, A.vscale, x, y, A.radius, A.minvar, out + 3 * center);
+    }
+}
+
+// The regressions of a row of pixels per block, eight lanes to a system (pixel, bandwidth).
+//
+// The normal equations are symmetric, and positive definite by their ridge of 1e-4, so they
+// are solved by symmetric elimination without pivoting, from the last variable to the first:
+// only the first coefficient is wanted, and it is what is left over (484 multiply-adds a
+// system instead of the 1,980 of Gauss-Jordan elimination). Lane l of a system holds columns l
+// and 8 + l of the augmented 12 x 15 matrix (columns 12-14: the colour channels); the
+// neighbours' features and colours come from a tile in shared memory that the block loads
+// once. All in FP64, fused multiply-adds. A system with a pivot below 1e-10 or a result that
+// is not finite (NaN or infinity in the buffers) goes to `list` and is solved as the
+// reference does (regression_half).
+//
+// Bound by the FP64 pipe (25 neighbours x 33 operations a lane). 960x540, both bandwidths of
+// one half 1.63 ms (6.68 with regression_half for every pixel), the last regression 0.91 ms
+// (3.35); against that solver the image moves by 1e-15.
+constexpr int kRegWarps = 8;
+constexpr int kRegTileMax = 48 * 1024;   // shared memory of a tile: up to radius 6 (pairs), 4 (single)
+__host__ __device__ constexpr int reg_pixels(bool pair) { return kRegWarps * (pair ? 2 : 4); }
+__host__ __device__ constexpr long long reg_tile_bytes(bool pair, long long radius)
+{
+    return (reg_pixels(pair) + 2 * radius) * (2 * radius + 1) * 14 * (long long)sizeof(double);
+}
+
+template <bool PAIR>
+__global__ void __launch_bounds__(32 * kRegWarps) k_regression(RegArgs A, unsigned* list, unsigned* list_n)
+{
+    extern __shared__ __align__(16) double s_tile[];
+    const Img I = A.I;
+    constexpr int TW = reg_pixels(PAIR);
+    const int R = A.radius, side = 2 * R + 1, K = side * side, cols = TW + 2 * R;
+    const int x0 = blockIdx.x * TW, y = blockIdx.y;
+    for (int i = threadIdx.x; i < cols * side * 14; i += blockDim.x) {
+        const int e = i / 14, f = i - 14 * e, ty = e / cols, tx = e - ty * cols;
+        const size_t s = (size_t)clampc(y + ty - R, I.h) * I.w + clampc(x0 + tx - R, I.w);
+        s_tile[i] = f < kF ? A.features[kF * s + f] : A.image[3 * s + (f - kF)];
+    }
+    __syncthreads();
+    const int lane = threadIdx.x & 31, l = lane & 7, g = lane >> 3;
+    const unsigned gmask = 0xffu << (8 * g);
+    const int px = (int)(threadIdx.x >> 5) * (PAIR ? 2 : 4) + (PAIR ? g >> 1 : g), x = x0 + px;
+    const bool second = PAIR && (g & 1);
+    if (x >= I.w) return;   // whole systems leave
+    const size_t npix = (size_t)I.w * I.h, pix = (size_t)y * I.w + x;
+    const double bw = second ? A.bw2 : A.bw1;
+    const double* center = s_tile + 14 * (R * cols + px + R);
+    double fc[kF];
+#pragma unroll
+    for (int f = 0; f < kF; f++) fc[f] = center[f];
+    const int ia = l > 0 ? l - 1 : 0, ib = l < 7 ? 7 + l : 13;   // this lane's columns in a tile entry
+    const double ca = center[ia], cb = l < 4 ? center[ib] : 0.0;
+    double MA[8], MB[kR];
+#pragma unroll
+    for (int r = 0; r < 8; r++) MA[r] = r == l ? 1e-4 : 0.0;
+#pragma unroll
+    for (int r = 0; r < kR; r++) MB[r] = r == 8 + l ? 1e-4 : 0.0;   // rows 8..11 of columns 8..11
+    double wreg = 0.0;
+    int k = 0;
+    for (int oy = 0; oy < side; oy++)
+        for (int ox = 0; ox < side; ox++, k++) {
+            if ((k & 7) == 0) {   // weights of neighbours k .. k + 7, one per lane
+                const int kk = k + l;
+                wreg = kk < K ? weight_from_distance(A.dist[(size_t)kk * npix + pix], bw, A.minvar) : 0.0;
+            }
+            const double wgt = __shfl_sync(gmask, wreg, k & 7, 8);
+            const double* n = s_tile + 14 * (oy * cols + px + ox);
+            const double2* n2 = reinterpret_cast<const double2*>(n);
+            double b[kR];
+            b[0] = 1.0;
+#pragma unroll
+            for (int q = 0; q < 6; q++) {
+                const double2 v = n2[q];
+                b[2 * q + 1] = v.x - fc[2 * q];
+                if (q < 5) b[2 * q + 2] = v.y - fc[2 * q + 1];
+            }
+            const double wa = l > 0 ? wgt * (n[ia] - ca) : wgt, wb = wgt * (n[ib] - cb);
+            MA[0] += wa;
+            MB[0] += wb;
+#pragma unroll
+            for (int r = 1; r < kR; r++) {
+                if (r < 8) MA[r] = fma(b[r], wa, MA[r]);
+                MB[r] = fma(b[r], wb, MB[r]);
+            }
+        }
+    bool ok = true;
+#pragma unroll
+    for (int p = kR - 1; p > 0; p--) {
+        const int src = p & 7;
+        const double piv = __shfl_sync(gmask, p < 8 ? MA[p < 8 ? p : 0] : MB[p], src, 8);
+        ok = ok && piv >= 1e-10;
+        const double inv = 1.0 / piv;
+        double col[kR], ra = p < 8 ? MA[p < 8 ? p : 0] : 0.0;
+#pragma unroll
+        for (int r = 0; r < p; r++) {
+            col[r] = __shfl_sync(gmask, p < 8 ? MA[r < 8 ? r : 0] : MB[r], src, 8);
+            if (p >= 8 && r == l) ra = col[r];   // row p of column l: row l of column p
+        }
+        const double ta = -(ra * inv), tb = -(MB[p] * inv);
+#pragma unroll
+        for (int r = 0; r < p; r++) {
+            if (r < 8) MA[r] = fma(col[r], ta, MA[r]);
+            MB[r] = fma(col[r], tb, MB[r]);
+        }
+    }
+    const double last = __shfl_sync(gmask, MA[0], 0, 8);
+    const double v = MB[0] / last;
+    const bool colour = l >= 4 && l < 7;
+    ok = ok && last >= 1e-10 && (!colour || isfinite(v));
+    if (__all_sync(gmask, ok)) {
+        double* out = second ? A.out2 : A.out1;
+        if (colour) out[3 * pix + (l - 4)] = v;
+    } else if (l == 0) {
+        list[atomicAdd(list_n, 1u)] = (unsigned)(pix << 1) | (second ? 1u : 0u);
     }
 }
 
@@ -497,16 +624,31 @@ void run_device(const double* ca, const double* cb, const double* cv, const doub
     double* ra2 = B.get(3 * n);
     double* rb1 = B.get(3 * n);
     double* rb2 = B.get(3 * n);
-    const unsigned rgrid_pair = (unsigned)((n * 32 + 127) / 128), rgrid_single = (unsigned)((((n + 1) / 2) * 32 + 127) / 128);
     const size_t K = (size_t)(2 * s.regression_radius + 1) * (2 * s.regression_radius + 1);
     double* dist = B.get(K * n);
     const unsigned dgrid = (unsigned)((K * n + 255) / 256);
+    // systems left to regression_half: at most two per pixel, 32 bits each; and their number
+    unsigned* list = reinterpret_cast<unsigned*>(B.get(n));
+    unsigned* list_n = reinterpret_cast<unsigned*>(B.get(1));
+    auto regress = [&](const RegArgs& A) {
+        const bool pair = A.bw2 >= 0.0;
+        k_patch_dist<<<dgrid, 256, 0, st>>>(A, dist);
+        const long long tile = reg_tile_bytes(pair, A.radius);
+        if (tile > kRegTileMax || n >= (1ull << 31)) {   // a window too wide for a tile
+            const size_t warps = pair ? n : (n + 1) / 2;
+            k_regression_warp<<<(unsigned)((warps * 32 + 127) / 128), 128, 0, st>>>(A, nullptr, nullptr);
+            return;
+        }
+        NCK(cudaMemsetAsync(list_n, 0, sizeof(unsigned), st));
+        const dim3 grid((unsigned)((width + reg_pixels(pair) - 1) / reg_pixels(pair)), (unsigned)height);
+        if (pair) k_regression<true><<<grid, 32 * kRegWarps, (size_t)tile, st>>>(A, list, list_n);
+        else k_regression<false><<<grid, 32 * kRegWarps, (size_t)tile, st>>>(A, list, list_n);
+        k_regression_warp<<<148, 128, 0, st>>>(A, list, list_n);
+    };
     RegArgs A{I, fa, pfb, cv, 2.0, s.regression_radius, s.patch_radius, s.min_variance, 0.5, 1.0, ra1, ra2, dist};
-    k_patch_dist<<<dgrid, 256, 0, st>>>(A, dist);
-    k_regression_warp<<<rgrid_pair, 128, 0, st>>>(A);
+    regress(A);
     RegArgs Bb{I, fb, pfa, cv, 2.0, s.regression_radius, s.patch_radius, s.min_variance, 0.5, 1.0, rb1, rb2, dist};
-    k_patch_dist<<<dgrid, 256, 0, st>>>(Bb, dist);
-    k_regression_warp<<<rgrid_pair, 128, 0, st>>>(Bb);
+    regress(Bb);
     // MSE, filtered; selection, filtered (guide: the averaged colour, undoubled variance)
     double* m1 = B.get(n);
     double* m2 = B.get(n);
@@ -523,8 +665,7 @@ void run_device(const double* ca, const double* cb, const double* cv, const doub
     double* fv = B.get(n);
     k_combine<<<grd, blk, 0, st>>>(I, s1, s2, fm1, fm2, ra1, ra2, rb1, rb2, pfa, pfb, s.min_variance, comb, ff, fv);
     RegArgs C{I, comb, ff, fv, 1.0, s.regression_radius, s.patch_radius, s.min_variance, 1.0, -1.0, d_out, nullptr, dist};
-    k_patch_dist<<<dgrid, 256, 0, st>>>(C, dist);
-    k_regression_warp<<<rgrid_single, 128, 0, st>>>(C);
+    regress(C);
     NCK(cudaGetLastError());
 }
 

@@ -32,9 +32,17 @@ ShadeKernel shade_kernel(int mode, int part, bool cold)
     if (mode == 2) return shade_kernel_cached();
     if (mode == 3) return cold ? k_shade<3, SHADE_ALL, true> : k_shade<3, SHADE_ALL, false>;
     if (part == SHADE_MISSES) return cold ? k_shade_misses<0, true> : k_shade_misses<0, false>;
-    if (mode == 1) return part == SHADE_HITS ? k_shade<1, SHADE_HITS, true> : k_shade<1, SHADE_ALL, true>;
-    if (cold) return part == SHADE_HITS ? k_shade<0, SHADE_HITS, true> : k_shade<0, SHADE_ALL, true>;
-    return part == SHADE_HITS ? k_shade<0, SHADE_HITS, false> : k_shade<0, SHADE_ALL, false>;
+    if (mode == 1)
+        return part == SHADE_HITS       ? k_shade<1, SHADE_HITS, true>
+               : part == SHADE_FEATURES ? k_shade<1, SHADE_FEATURES, true>
+                                        : k_shade<1, SHADE_ALL, true>;
+    if (cold)
+        return part == SHADE_HITS       ? k_shade<0, SHADE_HITS, true>
+               : part == SHADE_FEATURES ? k_shade<0, SHADE_FEATURES, true>
+                                        : k_shade<0, SHADE_ALL, true>;
+    return part == SHADE_HITS       ? k_shade<0, SHADE_HITS, false>
+           : part == SHADE_FEATURES ? k_shade<0, SHADE_FEATURES, false>
+                                    : k_shade<0, SHADE_ALL, false>;
 }
 
 }  // namespace luz

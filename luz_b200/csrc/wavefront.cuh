@@ -532,8 +532,9 @@ __device__ __forceinline__ void cache_inputs(const WaveArgs& w, const Hit& h, co
 
 // MODE 0: plain; 1: with the caustic photon map; 2: radiance-cache render;
 // 3: adjoint (gradient) passes. PART: the paths the kernel shades, SHADE_ALL of them, or
-// those that hit something or missed only (k_shade_hits, k_shade_misses).
-enum ShadePart : int { SHADE_ALL = 0, SHADE_HITS = 1, SHADE_MISSES = 2 };
+// those that hit something or missed only, or all of them with their NFOR features stored
+// (the first bounce of a render that asks for them).
+enum ShadePart : int { SHADE_ALL = 0, SHADE_HITS = 1, SHADE_MISSES = 2, SHADE_FEATURES = 3 };
 // COLD: the scene may hold what few scenes do (shade_cold); without it the kernel carries
 // neither that code nor the registers its calls take from the rest.
 template <int MODE, int PART, bool COLD>
@@ -637,7 +638,7 @@ static __device__ void shade_path(const DScene& S, const WaveArgs& w, const Path
         } else {
             sky = f3(S.k.background) * env_mis;
         }
-        if (COLD && bounce == 0 && w.nfor) store_miss_features(P, p, sky);   // env_mis is 1 at bounce 0
+        if (PART == SHADE_FEATURES) store_miss_features(P, p, sky);   // env_mis is 1 at bounce 0
         F3 contrib = thr * sky;
         if (bounce > 0 && S.k.has_constant_background_light) contrib = clamp_bg_miss(S, contrib);
         rad = rad + clamp_ray_color(contrib);
@@ -656,7 +657,7 @@ static __device__ void shade_path(const DScene& S, const WaveArgs& w, const Path
             mp = &m_res;
         }
         const GMaterial& m = *mp;
-        if (COLD && bounce == 0 && w.nfor) store_hit_features(S, P, p, h, m);
+        if (PART == SHADE_FEATURES) store_hit_features(S, P, p, h, m);
         if (COLD && bounce == 0 && S.k.sky == 2) {   // compositePrimaryAtmosphereSegment (ColorHelper.cpp:645-659)
             double ao[3], ad[3];
             atmos_ray(w, P, p, bounce, ray, ao, ad);
