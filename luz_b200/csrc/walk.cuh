@@ -487,8 +487,11 @@ constexpr int kLeafGroupMax = (F & TF_INSTANCE) ? LUZ_LEAF_GROUP_MAX_INST : LUZ_
 
 // Runs the walks of a warp's lanes to their ends; every lane of the warp calls it (a lane
 // without a ray with its state at WS_DONE). Node steps run while at least half of the live
-// lanes wait at one; then each other kind that some lane waits at runs once. SCENES: the
-// lanes' scenes may differ.
+// lanes wait at one; then each other kind that some lane waits at runs once. With instances
+// the lanes spread over leaves, top-level nodes and objects, and only the kind that most of
+// them wait at runs (leaves before top-level nodes before objects at equal numbers): 1e5
+// instances at 8 spp 198.4 -> 185.5 ms, the Cornell box 4.98 -> 4.91 ms (spheres without
+// instances 1.38 -> 1.42 ms, so not there). SCENES: the lanes' scenes may differ.
 template <bool SCENES, uint32_t F, bool ANY, bool COUNT, class VS>
 __device__ __forceinline__ void walk_warp(const DScene& S, Walk<F, ANY, COUNT, VS>& w, WorldRays* wr, VS& vs)
 {
@@ -502,7 +505,16 @@ __device__ __forceinline__ void walk_warp(const DScene& S, Walk<F, ANY, COUNT, V
             __syncwarp();
         }
         const unsigned leaves = __ballot_sync(full, w.state == WS_LEAF);
-        if (leaves) {
+        const unsigned objects = __ballot_sync(full, w.state == WS_OBJECT);
+        bool do_leaf = leaves != 0, do_object = objects != 0, do_top = true;
+        if constexpr ((F & TF_INSTANCE) != 0) {
+            const int n_leaf = __popc(leaves), n_object = __popc(objects),
+                      n_top = __popc(__ballot_sync(full, w.state == WS_TOP));
+            do_leaf = n_leaf > 0 && n_leaf >= max(n_top, n_object);
+            do_top = !do_leaf && n_top > 0 && n_top >= n_object;
+            do_object = !do_leaf && !do_top;
+        }
+        if (do_leaf) {
             if (__popc(leaves) > kLeafGroupMax<F>) {
                 if (w.state == WS_LEAF) w.leaf_step(S, wr);
             } else {
@@ -510,9 +522,11 @@ __device__ __forceinline__ void walk_warp(const DScene& S, Walk<F, ANY, COUNT, V
             }
             __syncwarp();
         }
-        if (__any_sync(full, w.state == WS_OBJECT || w.state == WS_TOP)) {
+        if (do_object) {
             if (w.state == WS_OBJECT) w.object_step(S, wr, vs);
             __syncwarp();
+        }
+        if (do_top) {
             if (w.state == WS_TOP) w.top_step(S);
             __syncwarp();
         }
