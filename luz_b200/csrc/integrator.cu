@@ -2077,6 +2077,19 @@ int do_adjoint_backward(luz_gpu_scene* s, const LuzRenderParams* p, int32_t text
     const int s_wave = (int)std::min<int64_t>(p->spp, n_wave);
     const int64_t pix_wave = std::max<int64_t>(1, std::min<int64_t>(npix, n_wave / s_wave));
     w.adj_rough = rough ? D.get<AdjRough>(pix_wave * s_wave, st) : nullptr;
+    // Albedo: one pass records each visit of the texture, and the gradients are added when
+    // the paths have ended; no path is traced twice. Visits beyond kAdjVisits per path (the
+    // textured Cornell box has 0.5) send their wave through the two passes instead.
+    constexpr int64_t kAdjVisits = 2;
+    const int64_t visits = kAdjVisits * pix_wave * s_wave;
+    AdjVertex* vertices = nullptr;
+    if (!rough) try {
+            vertices = D.raw<AdjVertex>(visits, st);
+        } catch (const Status&) {   // no room for them: two passes
+            (void)cudaGetLastError();
+        }
+    w.adj_count = D.get<unsigned long long>(1, st);
+    w.adj_cap = (unsigned long long)visits;
     CK(cudaMemcpyAsync(s->dds, &s->ds, sizeof(DScene), cudaMemcpyHostToDevice, st));
     CK(cudaEventRecord(s->ev0, st));
     StageTimer T0;
@@ -2091,12 +2104,34 @@ int do_adjoint_backward(luz_gpu_scene* s, const LuzRenderParams* p, int32_t text
             w.s_count = sc;
             w.n = pc * sc;
             const unsigned grid = (unsigned)((w.n + kBlock - 1) / kBlock);
+            if (vertices) {
+                w.adjoint = 1;
+                w.adj_vertices = vertices;
+                CK(cudaMemsetAsync(s->ctrl, 0, sizeof(Ctrl), st));
+                CK(cudaMemsetAsync(w.adj_count, 0, sizeof(unsigned long long), st));
+                k_raygen<<<grid, kBlock, 0, st>>>(w, s->pb, s->ctrl);
+                launch_bounces(s, w, st, launches, T0, 3, s->pb, s->ctrl);
+                unsigned long long* const seen = s->status_host;
+                CK(cudaMemcpyAsync(seen, w.adj_count, sizeof(*seen), cudaMemcpyDeviceToHost, st));
+                CK(cudaStreamSynchronize(st));
+                launches++;
+                w.adj_vertices = nullptr;
+                if (*seen <= w.adj_cap) {
+                    waves++;
+                    if (*seen == 0) continue;
+                    w.adj_vertices = vertices;
+                    adjoint_vertices_kernel()<<<(unsigned)std::min<int64_t>((int64_t)(*seen + 127) / 128, 64 * s->sms), 128, 0, st>>>(
+                        s->dds, w, s->pb);
+                    launches++;
+                    continue;
+                }
+            }
             for (int pass = 0; pass < 2; pass++) {   // 0: radiance of every path; 1: replay with gradients
                 w.adjoint = pass;
                 CK(cudaMemsetAsync(s->ctrl, 0, sizeof(Ctrl), st));
                 if (pass == 1 && rough) CK(cudaMemsetAsync(w.adj_rough, 0, sizeof(AdjRough) * (std::size_t)w.n, st));
                 k_raygen<<<grid, kBlock, 0, st>>>(w, s->pb, s->ctrl);
-                launch_bounces(s, w, st, launches, T0, 3, s->pb, s->ctrl);
+                launch_bounces(s, w, st, launches, T0, pass == 0 ? 0 : 3, s->pb, s->ctrl);
                 launches++;
                 if (pass == 0) {
                     k_path_color<<<grid, kBlock, 0, st>>>(w, s->pb);

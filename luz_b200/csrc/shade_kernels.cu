@@ -22,6 +22,21 @@
 
 namespace luz {
 
+// The gradients of a wave's visits of the differentiated texture, its paths ended.
+__global__ void k_adjoint_vertices(const DScene* __restrict__ Sp, WaveArgs w, PathBuf P)
+{
+    const DScene& S = *Sp;
+    const unsigned long long n = min(*w.adj_count, w.adj_cap), step = (unsigned long long)gridDim.x * blockDim.x;
+    for (unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += step) {
+        const AdjVertex v = w.adj_vertices[i];
+        const float4 r = P.rad[v.path], a = P.pend0[v.path], b = P.pend1[v.path];
+        const F3 L = (F3{r.x, r.y, r.z} + F3{a.x, a.y, a.z}) + F3{b.x, b.y, b.z};
+        adjoint_texture(S, w, P.pixel[v.path], L, v.u, v.v, F3{v.before[0], v.before[1], v.before[2]});
+    }
+}
+
+AdjointVerticesKernel adjoint_vertices_kernel() { return k_adjoint_vertices; }
+
 BatchShadeKernel batch_shade_kernel(int mode, bool cold)
 {
     return mode == 1 ? k_shade_batch<1, true> : cold ? k_shade_batch<0, true> : k_shade_batch<0, false>;

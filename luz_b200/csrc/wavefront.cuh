@@ -64,6 +64,14 @@ struct AdjRough {
     uint32_t active;
 };
 
+// A path's visit of the differentiated albedo texture: the radiance it had gathered before
+// the vertex, and where the texture was read. Its gradient waits for the path's end.
+struct AdjVertex {
+    float before[3];
+    float u, v;
+    uint32_t path;
+};
+
 struct WaveArgs {
     int32_t width, height;
     uint32_t seed, stream;
@@ -83,6 +91,9 @@ struct WaveArgs {
     int32_t grad_texture;         // texture whose texel gradient is accumulated
     int32_t grad_kind;            // 0: Lambertian albedo texture; 1: Metal roughness texture (red channel)
     AdjRough* adj_rough;          // grad_kind 1: one record per path
+    AdjVertex* adj_vertices;      // grad_kind 0: the wave's visits of the texture, adj_cap at most (NULL: a
+    unsigned long long* adj_count;   // replay adds their gradients, with the paths' radiance known), and their
+    unsigned long long adj_cap;   // number
     int32_t grad_emission;        // replay: gradient with respect to each light's emitted radiance
     double* grad_light;           // kEmissionReplicas copies of light_count * 3 (summed on the host)
     int32_t* pend_light;          // per path: light of the pending light sample, -1 = none
@@ -456,13 +467,11 @@ __device__ __forceinline__ void density_add(const DScene& S, const WaveArgs& w, 
 // per channel, zero where the clamp is active. The pixel's film is the mean of
 // cleanColor(L) over its samples, so each path adds adj(pixel) / spp times that.
 // Russian roulette's survival probability is held fixed (not differentiated).
-static __device__ __noinline__ void adjoint_texture(const DScene& S, const WaveArgs& w, const PathBuf& P, uint32_t p,
-                                             const Hit& h, F3 before)
+static __device__ __noinline__ void adjoint_texture(const DScene& S, const WaveArgs& w, uint32_t pix, F3 L, float hu, float hv,
+                                             F3 before)
 {
-    const float4 L = P.color[p];
-    const uint32_t pix = P.pixel[p];
     const GTexture T = S.textures[w.grad_texture];
-    const float u = wrap01f(h.u), v = wrap01f(h.v);
+    const float u = wrap01f(hu), v = wrap01f(hv);
     const float x = u * (float)(T.width - 1);
     const float y = (1.0f - v) * (float)(T.height - 1);
     const int x0 = (int)floorf(x), y0 = (int)floorf(y);
@@ -731,8 +740,15 @@ static __device__ void shade_path(const DScene& S, const WaveArgs& w, const Path
                 }
             }
         }
-        if (MODE == 3 && w.adjoint && w.grad_kind == 0 && m.type == MT_LAMBERTIAN && m.texture == w.grad_texture)
-            adjoint_texture(S, w, P, p, h, rad);
+        if (MODE == 3 && w.adjoint && w.grad_kind == 0 && m.type == MT_LAMBERTIAN && m.texture == w.grad_texture) {
+            if (w.adj_vertices) {
+                const unsigned long long i = atomicAdd(w.adj_count, 1ull);
+                if (i < w.adj_cap) w.adj_vertices[i] = AdjVertex{{rad.x, rad.y, rad.z}, h.u, h.v, p};
+            } else {
+                const float4 L = P.color[p];
+                adjoint_texture(S, w, pix, F3{L.x, L.y, L.z}, h.u, h.v, rad);
+            }
+        }
         const bool rough_grad =
             MODE == 3 && w.adjoint && w.grad_kind == 1 && m.type == MT_METAL && m.rtexture == w.grad_texture;
         if (rough_grad) {
@@ -890,6 +906,10 @@ __device__ __forceinline__ F3 clean(F3 c)   // cleanColor (Threads.cpp:122-137)
 using ShadeKernel = void (*)(const DScene*, WaveArgs, PathBuf, Ctrl*, int);
 ShadeKernel shade_kernel(int mode, int part, bool cold);
 ShadeKernel shade_kernel_cached();   // k_shade<2>, in its own translation unit
+
+// k_adjoint_vertices (shade_kernels.cu, so that the texture lookup rounds as the replay's).
+using AdjointVerticesKernel = void (*)(const DScene*, WaveArgs, PathBuf);
+AdjointVerticesKernel adjoint_vertices_kernel();
 
 // Multi-scene waves: every path finds its segment in P.seg, the segment's WaveArgs
 // in segs and its scene in scenes[segs[seg].batch_scene]. Modes 0 and 1 as above.
