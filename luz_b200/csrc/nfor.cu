@@ -149,23 +149,6 @@ __global__ void k_prefilter(Img I, const double* image, const double* guide, con
     }
 }
 
-// patchDistance (NFOR.cpp:240-310): the clamped loop (equal to the unclamped one inside the image).
-__device__ double patch_distance(Img I, const double* guide, const double* var, double vscale, int x1, int y1, int x2,
-                                 int y2, int r, double minvar)
-{
-    if (x1 == x2 && y1 == y2) return 0.0;
-    double dist = 0.0;
-    unsigned n = 0;
-    for (int oy = -r; oy <= r; oy++)
-        for (int ox = -r; ox <= r; ox++) {
-            const int a = clampc(y1 + oy, I.h) * I.w + clampc(x1 + ox, I.w);
-            const int b = clampc(y2 + oy, I.h) * I.w + clampc(x2 + ox, I.w);
-            const double lv = (var[a] * vscale) + (var[b] * vscale) + minvar;
-            dist += cdist2(guide + 3 * a, guide + 3 * b) / lv;
-            n++;
-        }
-    return dist / (double)n;
-}
 __device__ __forceinline__ double weight_from_distance(double d, double bw, double minvar)
 {
     return exp(-d / fmax(minvar, bw * bw));
@@ -206,11 +189,87 @@ struct RegArgs {
     const double* dist;      // patch distances: (2 radius + 1)^2 rows of one double per pixel (k_patch_dist)
 };
 
-// patchDistance (NFOR.cpp:482-517) of every pixel to each neighbour of its
-// regression window, row k = (oy + radius) (2 radius + 1) + (ox + radius): the
-// terms summed in patch order, then divided by the patch size; 0 where the
-// clamped neighbour is the pixel itself. One thread per (neighbour, pixel).
-__global__ void k_patch_dist(RegArgs A, double* D)
+// patchDistance (NFOR.cpp:482-517) of pixel (x, y) to its clamped neighbour (sx, sy): the terms
+// summed in patch order, then divided by the patch size; 0 where they are the same pixel.
+__device__ double patch_dist_at(const RegArgs& A, int x, int y, int sx, int sy)
+{
+    if (sx == x && sy == y) return 0.0;
+    const Img I = A.I;
+    const int pw = 2 * A.patch + 1, P = pw * pw;
+    double d = 0.0;
+    for (int t = 0; t < P; t++) {
+        const int py = t / pw - A.patch, px = t % pw - A.patch;
+        const int a = clampc(y + py, I.h) * I.w + clampc(x + px, I.w);
+        const int b = clampc(sy + py, I.h) * I.w + clampc(sx + px, I.w);
+        const double lv = (A.var[a] * A.vscale) + (A.var[b] * A.vscale) + A.minvar;
+        d += cdist2(A.image + 3 * a, A.image + 3 * b) / lv;
+    }
+    return d / (double)P;
+}
+
+// The patch distances of every pixel to each neighbour of its window, row k = (oy + radius)
+// (2 radius + 1) + (ox + radius); WEIGHT: weight_from_distance with bandwidth 1 of them. A
+// block takes a tile of 32 x 8 pixels with its colours and variances in shared memory. For one
+// neighbour offset o the term of a patch position depends on the position alone, so the
+// block forms each term once, for the tile and its rim, and every pixel sums its own: 1.3
+// terms (each with a FP64 division, which bounds it) per pixel and offset instead of a patch
+// of 9. The sums take the terms in patch order, so each distance has the same bits. Where the
+// neighbour itself is clamped to the image the terms are others: patch_dist_at. 960x540,
+// radius 2: 0.24 ms (0.55 with nine terms a thread); the filters' weights (radius 3) 0.53 ms
+// once, and 0.06 ms a filter that reads them (0.82 ms a filter that formed them).
+constexpr int kDistW = 32, kDistH = 8;
+constexpr int kDistTileMax = 48 * 1024;
+__host__ __device__ constexpr long long dist_tile_bytes(long long radius, long long patch)
+{
+    return ((kDistW + 2 * (radius + patch)) * (kDistH + 2 * (radius + patch)) * 4
+            + (kDistW + 2 * patch) * (kDistH + 2 * patch)) * (long long)sizeof(double);
+}
+template <bool WEIGHT>
+__global__ void __launch_bounds__(kDistW* kDistH) k_patch_dist(RegArgs A, double* D)
+{
+    extern __shared__ __align__(16) double s_tile[];
+    const Img I = A.I;
+    const int R = A.radius, Q = A.patch, H = R + Q, side = 2 * R + 1, pw = 2 * Q + 1;
+    const int cols = kDistW + 2 * H, rows = kDistH + 2 * H, tcols = kDistW + 2 * Q, trows = kDistH + 2 * Q;
+    double* const terms = s_tile + 4 * cols * rows;
+    const int x0 = blockIdx.x * kDistW, y0 = blockIdx.y * kDistH, tid = threadIdx.x;
+    for (int i = tid; i < cols * rows; i += kDistW * kDistH) {
+        const int ty = i / cols, tx = i - ty * cols;
+        const size_t s = (size_t)clampc(y0 + ty - H, I.h) * I.w + clampc(x0 + tx - H, I.w);
+        for (int c = 0; c < 3; c++) s_tile[4 * i + c] = A.image[3 * s + c];
+        s_tile[4 * i + 3] = A.var[s];
+    }
+    const int lx = tid % kDistW, ly = tid / kDistW, x = x0 + lx, y = y0 + ly;
+    const bool inside = x < I.w && y < I.h;
+    const size_t npix = (size_t)I.w * I.h, pix = (size_t)y * I.w + x;
+    for (int k = 0; k < side * side; k++) {
+        const int ox = k % side - R, oy = k / side - R;
+        __syncthreads();   // the tile is loaded; the last offset's terms are read
+        if (ox != 0 || oy != 0)
+            for (int i = tid; i < tcols * trows; i += kDistW * kDistH) {
+                const int ty = i / tcols, tx = i - ty * tcols;
+                const double* a = s_tile + 4 * ((ty + R) * cols + tx + R);
+                const double* b = a + 4 * (oy * cols + ox);
+                const double lv = (a[3] * A.vscale) + (b[3] * A.vscale) + A.minvar;
+                terms[i] = cdist2(a, b) / lv;
+            }
+        __syncthreads();
+        if (!inside) continue;
+        double d = 0.0;
+        if (ox != 0 || oy != 0) {
+            if (x + ox >= 0 && x + ox < I.w && y + oy >= 0 && y + oy < I.h) {
+                for (int py = 0; py < pw; py++)
+                    for (int px = 0; px < pw; px++) d += terms[(ly + py) * tcols + lx + px];
+                d = d / (double)(pw * pw);
+            } else {
+                d = patch_dist_at(A, x, y, clampc(x + ox, I.w), clampc(y + oy, I.h));
+            }
+        }
+        D[(size_t)k * npix + pix] = WEIGHT ? weight_from_distance(d, 1.0, A.minvar) : d;
+    }
+}
+// The same, one thread per (neighbour, pixel), for windows too wide for a tile.
+__global__ void k_patch_dist_wide(RegArgs A, double* D)
 {
     const Img I = A.I;
     const long long npix = (long long)I.w * I.h;
@@ -220,20 +279,7 @@ __global__ void k_patch_dist(RegArgs A, double* D)
     const int k = (int)(idx / npix);
     const long long pix = idx % npix;
     const int x = (int)(pix % I.w), y = (int)(pix / I.w);
-    const int sx = clampc(x + (k % side - A.radius), I.w), sy = clampc(y + (k / side - A.radius), I.h);
-    double d = 0.0;
-    if (!(sx == x && sy == y)) {
-        const int pw = 2 * A.patch + 1, P = pw * pw;
-        for (int t = 0; t < P; t++) {
-            const int py = t / pw - A.patch, px = t % pw - A.patch;
-            const int a = clampc(y + py, I.h) * I.w + clampc(x + px, I.w);
-            const int b = clampc(sy + py, I.h) * I.w + clampc(sx + px, I.w);
-            const double lv = (A.var[a] * A.vscale) + (A.var[b] * A.vscale) + A.minvar;
-            d += cdist2(A.image + 3 * a, A.image + 3 * b) / lv;
-        }
-        d = d / (double)P;
-    }
-    D[idx] = d;
+    D[idx] = patch_dist_at(A, x, y, clampc(x + (k % side - A.radius), I.w), clampc(y + (k / side - A.radius), I.h));
 }
 
 // regressionPass (NFOR.cpp:674-738) / regressionPairPass (:740-831) with one
@@ -498,9 +544,10 @@ __global__ void k_mse(Img I, const double* ca, const double* cb, const double* f
 }
 
 // filterScalarMapPair (NFOR.cpp:833-901): patch radius 1, bandwidth 1. select != 0
-// filters the bandwidth-selection maps of a and b instead of a and b.
-__global__ void k_filter_pair(Img I, const double* a, const double* b, int select, const double* guide,
-                              const double* gvar, int radius, double minvar, double* oa, double* ob)
+// filters the bandwidth-selection maps of a and b instead of a and b. Both filters have the
+// same guide, hence the same weights: weight holds them (k_patch_dist<true>, as its rows).
+__global__ void k_filter_pair(Img I, const double* a, const double* b, int select, const double* weight, int radius,
+                              double* oa, double* ob)
 {
     const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
     if (x >= I.w || y >= I.h) return;
@@ -508,12 +555,12 @@ __global__ void k_filter_pair(Img I, const double* a, const double* b, int selec
     auto vb = [&](int s) { return select ? (b[s] <= a[s] ? 1.0 : 0.0) : b[s]; };
     double fa = 0.0, fb = 0.0, total = 0.0;
     const int center = y * I.w + x;
+    const size_t npix = (size_t)I.w * I.h;
+    const double* w = weight + center;
     for (int oy = -radius; oy <= radius; oy++)
-        for (int ox = -radius; ox <= radius; ox++) {
-            const int sx = clampc(x + ox, I.w), sy = clampc(y + oy, I.h);
-            const int s = sy * I.w + sx;
-            const double d = patch_distance(I, guide, gvar, 1.0, x, y, sx, sy, 1, minvar);
-            const double wgt = weight_from_distance(d, 1.0, minvar);
+        for (int ox = -radius; ox <= radius; ox++, w += npix) {
+            const int s = clampc(y + oy, I.h) * I.w + clampc(x + ox, I.w);
+            const double wgt = *w;
             fa += va(s) * wgt;
             fb += vb(s) * wgt;
             total += wgt;
@@ -625,14 +672,18 @@ void run_device(const double* ca, const double* cb, const double* cv, const doub
     double* rb1 = B.get(3 * n);
     double* rb2 = B.get(3 * n);
     const size_t K = (size_t)(2 * s.regression_radius + 1) * (2 * s.regression_radius + 1);
-    double* dist = B.get(K * n);
-    const unsigned dgrid = (unsigned)((K * n + 255) / 256);
+    constexpr int kFilterRadius = 3;
+    constexpr size_t kFilterWindow = (2 * kFilterRadius + 1) * (2 * kFilterRadius + 1);
+    double* dist = B.get((K > kFilterWindow ? K : kFilterWindow) * n);
+    const dim3 dgrid((unsigned)((width + kDistW - 1) / kDistW), (unsigned)((height + kDistH - 1) / kDistH));
     // systems left to regression_half: at most two per pixel, 32 bits each; and their number
     unsigned* list = reinterpret_cast<unsigned*>(B.get(n));
     unsigned* list_n = reinterpret_cast<unsigned*>(B.get(1));
     auto regress = [&](const RegArgs& A) {
         const bool pair = A.bw2 >= 0.0;
-        k_patch_dist<<<dgrid, 256, 0, st>>>(A, dist);
+        const long long dtile = dist_tile_bytes(A.radius, A.patch);
+        if (dtile <= kDistTileMax) k_patch_dist<false><<<dgrid, kDistW * kDistH, (size_t)dtile, st>>>(A, dist);
+        else k_patch_dist_wide<<<(unsigned)((K * n + 255) / 256), 256, 0, st>>>(A, dist);
         const long long tile = reg_tile_bytes(pair, A.radius);
         if (tile > kRegTileMax || n >= (1ull << 31)) {   // a window too wide for a tile
             const size_t warps = pair ? n : (n + 1) / 2;
@@ -657,8 +708,10 @@ void run_device(const double* ca, const double* cb, const double* cv, const doub
     double* s1 = B.get(n);
     double* s2 = B.get(n);
     k_mse<<<grd, blk, 0, st>>>(I, fa, fb, ra1, rb1, ra2, rb2, cv, m1, m2);
-    k_filter_pair<<<grd, blk, 0, st>>>(I, m1, m2, 0, col, cv, 3, s.min_variance, fm1, fm2);
-    k_filter_pair<<<grd, blk, 0, st>>>(I, fm1, fm2, 1, col, cv, 3, s.min_variance, s1, s2);
+    const RegArgs W{I, col, nullptr, cv, 1.0, kFilterRadius, 1, s.min_variance, 1.0, -1.0, nullptr, nullptr, nullptr};
+    k_patch_dist<true><<<dgrid, kDistW * kDistH, (size_t)dist_tile_bytes(kFilterRadius, 1), st>>>(W, dist);
+    k_filter_pair<<<grd, blk, 0, st>>>(I, m1, m2, 0, dist, kFilterRadius, fm1, fm2);
+    k_filter_pair<<<grd, blk, 0, st>>>(I, fm1, fm2, 1, dist, kFilterRadius, s1, s2);
     // blend, final features and variance, last regression
     double* comb = B.get(3 * n);
     double* ff = B.get(kF * n);

@@ -24,7 +24,7 @@ int luz_nfor_on_device(const double* color_a, const double* color_b, const doubl
 // synchronisation), gives all of it back when the last handle of the device is destroyed or
 // an allocation outside it fails, and orders reuse between streams and threads by the
 // streams' own dependencies.
-constexpr unsigned long long kScratchKeep = 2ull << 30;
+constexpr unsigned long long kScratchKeep = 3ull << 30;
 
 // The current device's scratch pool; on failure NULL, with the CUDA error in *err.
 cudaMemPool_t luz_scratch_pool(cudaError_t* err);

@@ -102,7 +102,7 @@ def buffers(w, h, seed):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("w,h,radius", [(1, 1, 2), (2, 3, 1), (16, 2, 2), (17, 9, 2), (33, 5, 4), (31, 7, 5), (20, 18, 6),
-                                        (18, 17, 7)])
+                                        (18, 17, 7), (64, 9, 3), (65, 8, 2)])
 def test_regression_equals_the_restatement(w, h, radius):
     b = buffers(w, h, 10 * w + h)
     out = native.nfor_denoise(b, regression_radius=radius)

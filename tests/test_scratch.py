@@ -51,7 +51,7 @@ def test_threads_share_the_pool():
 
 
 def test_the_last_handle_gives_the_memory_back():
-    """In a process of its own: a 960x540 denoise leaves at most 2 GiB in the pool, and the
+    """In a process of its own: a 960x540 denoise leaves at most 3 GiB in the pool, and the
     end of the last handle leaves what an idle process held before it (to 64 MiB)."""
     code = """
 import numpy as np, torch
@@ -68,7 +68,7 @@ held = free0 - torch.cuda.mem_get_info()[0]
 g.close()
 left = free0 - torch.cuda.mem_get_info()[0]
 print(held >> 20, left >> 20)
-assert (64 << 20) < held <= (2 << 30) + (64 << 20) and left <= (64 << 20), (held, left)
+assert (64 << 20) < held <= (3 << 30) + (64 << 20) and left <= (64 << 20), (held, left)
 """
     r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout + r.stderr
