@@ -341,9 +341,10 @@ int luz_gpu_scene_set_traversal_limits(luz_gpu_scene* scene, int32_t mesh_entrie
  *   staged_top_nodes:     1 = the trace kernels copy the breadth-first top of the scene's
  *                         largest collapsed mesh BVH (21 nodes) into shared memory per
  *                         block and read those nodes there;
- *   *_blocks_per_sm:      blocks per SM of the persistent closest-hit / any-hit grids and
- *                         of the shade grid (default: full occupancy; larger values are
- *                         capped at it);
+ *   *_blocks_per_sm:      blocks per SM of the persistent trace grid (extend: launches that
+ *                         hold closest-hit rays, with the shadow rays of the bounce before;
+ *                         shadow: launches of shadow rays alone) and of the shade grid
+ *                         (default: full occupancy; larger values are capped at it);
  *   sort_rays, lanes:     see the fields.
  * No counterpart in the reference (its worker count is Scene::setRenderingThreads). */
 typedef struct LuzTuneParams {

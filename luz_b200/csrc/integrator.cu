@@ -1,16 +1,17 @@
 // integrator.cu — wavefront path tracer for B200 (sm_100a) behind the C ABI.
 //
 // One render = waves of (pixel block x sample block) paths. Each wave runs
-//   raygen  -> [extend -> shade -> shadow] x (max_bounces + 1) -> accumulate
-// over SoA path state. Queues are compacted with warp ballots (one atomic per
-// warp); extend/shadow are persistent kernels whose warps fetch 32-ray batches
-// from a global counter, so warps that finish early steal the remaining work.
+//   raygen  -> [trace -> shade] x (max_bounces + 1) -> trace -> accumulate
+// over SoA path state; a trace launch takes the extension rays of its bounce and
+// the shadow rays of the one before. Queues are compacted with warp ballots (one
+// atomic per warp); the trace kernel is persistent, its warps fetch batches of rays
+// from global counters, so warps that finish early steal the remaining work.
 // Per-bounce counters live on the device; the host never waits inside a wave.
 //
 // The per-path arithmetic follows calculateLightRaysColor
 // (src/renderer/ColorHelper.cpp:1136-1326) step for step; NEE shadow tests are
-// deferred to the shadow kernel: shade stores each candidate contribution in a
-// per-path "pending" slot and the shadow kernel clears the slot when the ray is
+// deferred to the next trace launch: shade stores each candidate contribution in a
+// per-path "pending" slot and the trace kernel clears the slot when the ray is
 // occluded, which gives the same sum as the reference's inline test.
 #include <cub/device/device_radix_sort.cuh>
 #include <cuda_runtime.h>
@@ -54,7 +55,10 @@ __global__ void __launch_bounds__(kBlock) k_raygen(WaveArgs w, PathBuf P, Ctrl* 
 
 // ---------------------------------------------------------------------------- trace (closest and any hits)
 
-// Resident blocks per SM the register allocator is asked to allow.
+// Resident blocks per SM the register allocator is asked to allow, measured on one B200:
+// 8 blocks (64 registers) 214.8 ms on the 1080p glossy frame at 64 spp, 7 (72) 223.5, 9 (56)
+// 217.8, 10 224.7; with instances 6 (80) 203.7 ms on the 1e5-instance frame at 8 spp, 5 213.9,
+// 7 202.5 (and 2.97 instead of 2.80 ms on a 640x360 draft).
 #ifndef LUZ_TRACE_MIN_BLOCKS
 #define LUZ_TRACE_MIN_BLOCKS 8
 #endif
@@ -238,7 +242,7 @@ __global__ void __launch_bounds__(kBlock, (F & TF_INSTANCE) ? LUZ_TRACE_MIN_BLOC
 using TraceKernel = void (*)(DScene, WaveArgs, PathBuf, Ctrl*, int, int);
 // Indexed [count][features | staged]: TF_STAGED variants read the scene's top
 // collapsed nodes from shared memory (a tuning choice, off by default: on the
-// 1080p glossy frame they measured 2.5% slower, the nodes being L1-resident).
+// 1080p glossy frame at 64 spp 183.8 against 180.3 ms, the nodes being L1-resident).
 const TraceKernel kTraceKernels[2][8] = {
     {k_trace<0, false>, k_trace<1, false>, k_trace<2, false>, k_trace<3, false>,
      k_trace<4, false>, k_trace<5, false>, k_trace<6, false>, k_trace<7, false>},
@@ -1355,10 +1359,9 @@ bool shade_cold(const ScenePack& P)
 constexpr int64_t kMinLanePaths = int64_t(1) << 22;
 
 // Paths in flight per wave. A launch of the persistent trace kernels lasts at
-// least as long as its slowest warp's traversal, a tail of the order of half a
-// millisecond per bounce on incoherent rays; larger waves pay it fewer times per
-// frame (1080p glossy frame, 64 spp: 4 Mi paths 231.5, 8 Mi 305.6, 16 Mi 363.5,
-// 32 Mi 395.4-400.0, 64 Mi 414.5 Msamples/s, the image the same bit for bit).
+// least as long as its slowest warp's traversal; larger waves pay it fewer times per
+// frame (1080p glossy frame, 64 spp: 4 Mi paths 252.3, 16 Mi 194.6, 64 Mi 180.3 ms, the image
+// the same bit for bit).
 // Path state is 268 B per path (18 GB at 64 Mi, a tenth of the B200's HBM) and
 // stays allocated with the scene handle.
 constexpr int64_t kWaveTarget = int64_t(1) << 26;

@@ -7,9 +7,9 @@
 
 namespace luz {
 
-ShadeKernel shade_kernel_cached()
+ShadeKernel shade_kernel_cached(bool cold)
 {
-    return k_shade<2, SHADE_ALL, true>;
+    return cold ? k_shade<2, SHADE_ALL, true> : k_shade<2, SHADE_ALL, false>;
 }
 
 }  // namespace luz

@@ -44,7 +44,7 @@ BatchShadeKernel batch_shade_kernel(int mode, bool cold)
 
 ShadeKernel shade_kernel(int mode, int part, bool cold)
 {
-    if (mode == 2) return shade_kernel_cached();
+    if (mode == 2) return shade_kernel_cached(cold);
     if (mode == 3) return cold ? k_shade<3, SHADE_ALL, true> : k_shade<3, SHADE_ALL, false>;
     if (part == SHADE_MISSES) return cold ? k_shade_misses<0, true> : k_shade_misses<0, false>;
     if (mode == 1)

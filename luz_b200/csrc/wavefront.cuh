@@ -37,8 +37,7 @@ struct PathBuf {
     int2* sh_x;        // source primitive excluded from the shadow ray
     float4* color;     // per-path final colour
     float4* feat;      // NFOR primary-vertex features 2..10, 3 float4 per path (NULL unless requested)
-    uint32_t* bins;    // kShadeClasses segments of bin_stride paths, filled by extend in hit-class order
-                       // (NULL: shade reads the extension queue as it is)
+    uint32_t* bins;    // kShadeClasses segments of bin_stride paths, filled by the trace stage in hit-class order
     uint32_t bin_stride;
     uint32_t* seg;     // multi-scene waves: the wave segment (scene) of each path; NULL otherwise
     uint32_t* sort_keys;   // coherence sort of the extension queue (tuning): key per queue entry,
@@ -905,7 +904,7 @@ __device__ __forceinline__ F3 clean(F3 c)   // cleanColor (Threads.cpp:122-137)
 // caustic estimate, 2 radiance-cache render, 3 adjoint replay.
 using ShadeKernel = void (*)(const DScene*, WaveArgs, PathBuf, Ctrl*, int);
 ShadeKernel shade_kernel(int mode, int part, bool cold);
-ShadeKernel shade_kernel_cached();   // k_shade<2>, in its own translation unit
+ShadeKernel shade_kernel_cached(bool cold);   // k_shade<2>, in its own translation unit
 
 // k_adjoint_vertices (shade_kernels.cu, so that the texture lookup rounds as the replay's).
 using AdjointVerticesKernel = void (*)(const DScene*, WaveArgs, PathBuf);
