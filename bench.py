@@ -143,11 +143,11 @@ def measured_peak():
     return 6650.0, "fallback"
 
 
-PROFILE_SUMMARY = os.path.join(ROOT, "profiles", "k_extend_counters_mesh_glossy.md")
+PROFILE_SUMMARY = os.path.join(ROOT, "profiles", "k_trace_counters_mesh_glossy.md")
 
 
 def profile_counters():
-    """Per-extension-ray ncu figures of k_extend from the committed summary: DRAM bytes,
+    """Per-extension-ray ncu figures of k_trace from the committed summary: DRAM bytes,
     L2 bytes (lts__t_bytes), L2 throughput as a fraction of its peak
     (lts__throughput.avg.pct_of_peak_sustained_elapsed / 100) and active lanes per
     warp instruction (smsp__thread_inst_executed_per_inst_executed)."""
@@ -377,14 +377,14 @@ def run_ours(args):
                "clocks": clk,
                "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                             "frac": (achieved / peak) if achieved else None, "traffic": traffic,
-                            "kernel": "k_extend (closest-hit traversal)", "peak_kind": peak_kind,
+                            "kernel": "k_trace (closest-hit traversal, launched alone)", "peak_kind": peak_kind,
                             "algorithmic_bytes_per_ray": alg_bytes / max(1.0, ext_rays),
                             "bytes_formula": "64 x binary node visits + 48 x triangle tests + 32 x top-level "
                                              "records + 52 per ray",
                             "rays_per_launch": rays_per_launch,
                             "launch_ms": launch_ms,
                             "traffic_source": "ncu dram bytes per extension ray x rays per launch "
-                                              "(profiles/k_extend_counters_mesh_glossy.md)",
+                                              "(profiles/k_trace_counters_mesh_glossy.md)",
                             "l2_gbs": l2_gbs, "l2_frac": pc.get("l2_frac"),
                             "l2_source": "ncu lts__t_bytes per extension ray x rays per launch / live launch "
                                          "time; l2_frac = lts__throughput pct of peak (same summary)",
