@@ -2081,8 +2081,9 @@ int do_adjoint_backward(luz_gpu_scene* s, const LuzRenderParams* p, int32_t text
     const int64_t pix_wave = std::max<int64_t>(1, std::min<int64_t>(npix, n_wave / s_wave));
     w.adj_rough = rough ? D.get<AdjRough>(pix_wave * s_wave, st) : nullptr;
     // Albedo: one pass records each visit of the texture, and the gradients are added when
-    // the paths have ended; no path is traced twice. Visits beyond kAdjVisits per path (the
-    // textured Cornell box has 0.5) send their wave through the two passes instead.
+    // the paths have ended; no path is traced twice. In a wave with more than kAdjVisits visits
+    // per path (the textured Cornell box has 0.5) that pass serves as the first of the two that
+    // roughness takes: it leaves every path's radiance, and a replay adds the gradients.
     constexpr int64_t kAdjVisits = 2;
     const int64_t visits = kAdjVisits * pix_wave * s_wave;
     AdjVertex* vertices = nullptr;
@@ -2107,42 +2108,41 @@ int do_adjoint_backward(luz_gpu_scene* s, const LuzRenderParams* p, int32_t text
             w.s_count = sc;
             w.n = pc * sc;
             const unsigned grid = (unsigned)((w.n + kBlock - 1) / kBlock);
-            if (vertices) {
-                w.adjoint = 1;
-                w.adj_vertices = vertices;
+            // Both passes run the gradient kernel: another instantiation may round a decision of
+            // a path otherwise, and the replay has to be of the path whose radiance was taken.
+            auto trace = [&](int replay) {
+                w.adjoint = replay;
                 CK(cudaMemsetAsync(s->ctrl, 0, sizeof(Ctrl), st));
-                CK(cudaMemsetAsync(w.adj_count, 0, sizeof(unsigned long long), st));
                 k_raygen<<<grid, kBlock, 0, st>>>(w, s->pb, s->ctrl);
                 launch_bounces(s, w, st, launches, T0, 3, s->pb, s->ctrl);
+                launches++;
+            };
+            if (vertices) {
+                w.adj_vertices = vertices;
+                CK(cudaMemsetAsync(w.adj_count, 0, sizeof(unsigned long long), st));
+                trace(1);
                 unsigned long long* const seen = s->status_host;
                 CK(cudaMemcpyAsync(seen, w.adj_count, sizeof(*seen), cudaMemcpyDeviceToHost, st));
                 CK(cudaStreamSynchronize(st));
-                launches++;
-                w.adj_vertices = nullptr;
                 if (*seen <= w.adj_cap) {
                     waves++;
                     if (*seen == 0) continue;
-                    w.adj_vertices = vertices;
                     adjoint_vertices_kernel()<<<(unsigned)std::min<int64_t>((int64_t)(*seen + 127) / 128, 64 * s->sms), 128, 0, st>>>(
                         s->dds, w, s->pb);
                     launches++;
                     continue;
                 }
+                w.adj_vertices = nullptr;
+            } else {
+                trace(0);
             }
-            for (int pass = 0; pass < 2; pass++) {   // 0: radiance of every path; 1: replay with gradients
-                w.adjoint = pass;
-                CK(cudaMemsetAsync(s->ctrl, 0, sizeof(Ctrl), st));
-                if (pass == 1 && rough) CK(cudaMemsetAsync(w.adj_rough, 0, sizeof(AdjRough) * (std::size_t)w.n, st));
-                k_raygen<<<grid, kBlock, 0, st>>>(w, s->pb, s->ctrl);
-                launch_bounces(s, w, st, launches, T0, pass == 0 ? 0 : 3, s->pb, s->ctrl);
+            k_path_color<<<grid, kBlock, 0, st>>>(w, s->pb);
+            launches++;
+            if (rough) CK(cudaMemsetAsync(w.adj_rough, 0, sizeof(AdjRough) * (std::size_t)w.n, st));
+            trace(1);
+            if (rough) {
+                k_adjoint_rough_finish<<<grid, kBlock, 0, st>>>(s->ds, w, s->pb);
                 launches++;
-                if (pass == 0) {
-                    k_path_color<<<grid, kBlock, 0, st>>>(w, s->pb);
-                    launches++;
-                } else if (rough) {
-                    k_adjoint_rough_finish<<<grid, kBlock, 0, st>>>(s->ds, w, s->pb);
-                    launches++;
-                }
             }
             waves++;
         }
