@@ -315,8 +315,9 @@ int luz_pack_array(const luz_scene_pack* pack, const char* name, const void** da
 int luz_gpu_scene_create(const LuzSceneDesc* desc, int32_t device, luz_gpu_scene** out);
 int luz_gpu_scene_destroy(luz_gpu_scene* scene);
 int luz_gpu_scene_info(const luz_gpu_scene* scene, LuzSceneInfo* info);
-/* Caps the path state (the SoA arrays of one wave, 268 bytes per path, 316
- * with NFOR features) the handle may hold, in bytes; -1 restores the default,
+/* Caps the path state (the SoA arrays of one wave, 276 bytes per path, 324
+ * with NFOR features; an albedo gradient counts the 48 bytes per path of its
+ * recorded texture visits too) the handle may hold, in bytes; -1 restores the default,
  * a quarter of the device memory free (plus what the handle holds) when a
  * render allocates. Renders split into more, smaller waves under a lower cap
  * (the film does not depend on the wave size); when cudaMalloc refuses a wave

@@ -1235,15 +1235,16 @@ struct luz_gpu_scene {
     // large enough, else new ones of min(want, budget) paths. When cudaMalloc
     // refuses them (memory held by other work on the device) the request is
     // halved, down to kMinWavePaths, so the render runs in more, smaller waves
-    // (the image does not depend on the wave size). Returns the paths available.
-    int64_t reserve_paths(int64_t want, bool feat = false)
+    // (the image does not depend on the wave size). `extra`: bytes per path that
+    // the call itself allocates beside the path state; they count against the
+    // budget. Returns the paths available.
+    int64_t reserve_paths(int64_t want, bool feat = false, int64_t extra = 0)
     {
         want = std::max<int64_t>(1, want);
+        const int64_t per = kPathBytes + (feat ? kFeatBytes : 0) + extra;
         // buffers already held serve without asking the driver for its free memory
         // (cudaMemGetInfo costs host time on every render otherwise)
-        if (want <= cap && (!feat || pb.feat) && (path_budget < 0 || want * (kPathBytes + (feat ? kFeatBytes : 0)) <= path_budget))
-            return want;
-        const int64_t per = kPathBytes + (feat ? kFeatBytes : 0);
+        if (want <= cap && (!feat || pb.feat) && (path_budget < 0 || want * per <= path_budget)) return want;
         int64_t budget = path_budget;
         if (budget < 0) {
             size_t free_b = 0, total_b = 0;
@@ -1362,7 +1363,7 @@ constexpr int64_t kMinLanePaths = int64_t(1) << 22;
 // least as long as its slowest warp's traversal; larger waves pay it fewer times per
 // frame (1080p glossy frame, 64 spp: 4 Mi paths 252.3, 16 Mi 194.6, 64 Mi 180.3 ms, the image
 // the same bit for bit).
-// Path state is 268 B per path (18 GB at 64 Mi, a tenth of the B200's HBM) and
+// Path state is 276 B per path (18 GB at 64 Mi, a tenth of the B200's HBM) and
 // stays allocated with the scene handle.
 constexpr int64_t kWaveTarget = int64_t(1) << 26;
 // The cached render updates its cache once per wave; its default wave is 4 Mi
@@ -2076,7 +2077,9 @@ int do_adjoint_backward(luz_gpu_scene* s, const LuzRenderParams* p, int32_t text
     w.adj_rgb = d_adj;
     w.grad = d_grad;
     w.inv_spp = 1.0 / (double)p->spp;
-    const int64_t n_wave = s->reserve_paths(std::min<int64_t>(kWaveTarget, npix * (int64_t)p->spp));
+    constexpr int64_t kAdjVisits = 2;   // recorded visits per path (albedo)
+    const int64_t n_wave = s->reserve_paths(std::min<int64_t>(kWaveTarget, npix * (int64_t)p->spp), false,
+                                            rough ? 0 : kAdjVisits * (int64_t)sizeof(AdjVertex));
     const int s_wave = (int)std::min<int64_t>(p->spp, n_wave);
     const int64_t pix_wave = std::max<int64_t>(1, std::min<int64_t>(npix, n_wave / s_wave));
     w.adj_rough = rough ? D.get<AdjRough>(pix_wave * s_wave, st) : nullptr;
@@ -2084,7 +2087,6 @@ int do_adjoint_backward(luz_gpu_scene* s, const LuzRenderParams* p, int32_t text
     // the paths have ended; no path is traced twice. In a wave with more than kAdjVisits visits
     // per path (the textured Cornell box has 0.5) that pass serves as the first of the two that
     // roughness takes: it leaves every path's radiance, and a replay adds the gradients.
-    constexpr int64_t kAdjVisits = 2;
     const int64_t visits = kAdjVisits * pix_wave * s_wave;
     AdjVertex* vertices = nullptr;
     if (!rough) try {

@@ -52,3 +52,22 @@ def test_roughness_passes_run_the_same_kernels(side, spp):
         assert st.kernel_launches == 2 * trace_launches(bounces) + 2, st.kernel_launches
     finally:
         g.close()
+
+
+def test_recorded_visits_count_against_the_budget():
+    """A path takes 276 bytes of state and two records of 24 bytes: a budget of 4,096 paths'
+    state and records makes sixteen waves of 65,536 paths (fourteen if the state alone counted),
+    and the same gradient."""
+    side, spp, bounces = 128, 4, 3
+    w = scenes.cornell_textured(side, side, spp, bounces)
+    g = native.GpuScene(w.scene.build())
+    try:
+        p = native.params(side, side, spp, bounces, 9)
+        adj = np.random.default_rng(2).uniform(0.5, 1.5, (side, side, 3)).astype(np.float32)
+        ref, s0 = g.adjoint_backward(p, 0, adj, (32, 32, 3))
+        g.set_path_budget((276 + 48) * 4096)
+        got, s1 = g.adjoint_backward(p, 0, adj, (32, 32, 3))
+        assert s0.waves == 1 and s1.waves == side * side * spp // 4096, (s0.waves, s1.waves)
+        assert np.allclose(got, ref, rtol=1e-12, atol=1e-18)
+    finally:
+        g.close()
