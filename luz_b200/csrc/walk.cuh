@@ -280,9 +280,13 @@ struct Walk {
             }
             const bool mine = owner && (rank >> 2) == (r0 >> 2);
             const int gl = 8 * (rank & 3);
-            if constexpr (COUNT)
-                if (mine) n_tris += (ref & 7u) + 1u - (uint32_t)((uint32_t)(skip - (int32_t)((ref & 0x7fffffffu) >> 3)) <= (ref & 7u));
             const unsigned hits = __ballot_sync(full, ok);
+            if constexpr (COUNT)
+                if (mine) {   // as one after another: ANY ends at the first hit; the skipped triangle is not read
+                    const unsigned h8 = (hits >> gl) & 0xffu;
+                    const uint32_t last = ANY && h8 ? (uint32_t)__ffs(h8) - 1u : ref & 7u;
+                    n_tris += last + 1u - (uint32_t)((uint32_t)(skip - (int32_t)((ref & 0x7fffffffu) >> 3)) <= last);
+                }
             if constexpr (ANY) {
                 if (mine && ((hits >> gl) & 0xffu)) h.obj = obj;
             } else {
