@@ -1013,7 +1013,16 @@ template <class T> T* dalloc(std::size_t n)
 {
     void* p = nullptr;
     if (n == 0) n = 1;
-    CK(cudaMalloc(&p, n * sizeof(T)));
+    cudaError_t e = cudaMalloc(&p, n * sizeof(T));
+    if (e == cudaErrorMemoryAllocation) {   // once more with what the scratch pool holds idle
+        (void)cudaGetLastError();           // clears the allocation error
+        int device = 0;
+        CK(cudaGetDevice(&device));
+        luz_scratch_trim(device);
+        e = cudaMalloc(&p, n * sizeof(T));
+    }
+    if (e != cudaSuccess)
+        throw Status(LUZ_E_CUDA, "cudaMalloc of " + std::to_string(n * sizeof(T)) + " bytes: " + cudaGetErrorString(e));
     return static_cast<T*>(p);
 }
 template <class T> T* dupload(const std::vector<T>& v)
@@ -1024,17 +1033,15 @@ template <class T> T* dupload(const std::vector<T>& v)
 }
 
 // Device buffers of one call, from the device's scratch pool in the order of their stream,
-// given back to it on every exit path.
+// given back to it on every exit path; the call then waits for its stream (3 us: its work is
+// done), so that what the pool holds of it is idle and can be trimmed.
 struct DeviceScratch {
     std::vector<std::pair<void*, cudaStream_t>> ptrs;
     // n elements, not initialised
     template <class T> T* raw(int64_t n, cudaStream_t st)
     {
-        cudaError_t e = cudaSuccess;
-        const cudaMemPool_t pool = luz_scratch_pool(&e);
-        CK(e);
         void* p = nullptr;
-        CK(cudaMallocFromPoolAsync(&p, sizeof(T) * (std::size_t)std::max<int64_t>(n, 1), pool, st));
+        CK(luz_scratch_alloc(&p, sizeof(T) * (std::size_t)std::max<int64_t>(n, 1), st));
         ptrs.push_back({p, st});
         return static_cast<T*>(p);
     }
@@ -1048,6 +1055,8 @@ struct DeviceScratch {
     ~DeviceScratch()
     {
         for (auto& p : ptrs) cudaFreeAsync(p.first, p.second);
+        for (std::size_t i = 0; i < ptrs.size(); i++)
+            if (i == 0 || ptrs[i].second != ptrs[i - 1].second) cudaStreamSynchronize(ptrs[i].second);
     }
 };
 
@@ -1089,39 +1098,57 @@ std::vector<cudaMemPool_t> g_scratch;   // per device, created on first use, kep
 
 }  // namespace
 
-cudaMemPool_t luz_scratch_pool(cudaError_t* err)
+namespace {
+
+// The current device's scratch pool.
+cudaError_t scratch_pool(cudaMemPool_t* out, int* device)
 {
-    int device = 0;
-    *err = cudaGetDevice(&device);
-    if (*err != cudaSuccess) return nullptr;
+    cudaError_t e = cudaGetDevice(device);
+    if (e != cudaSuccess) return e;
     std::lock_guard<std::mutex> lock(g_scratch_mu);
-    if ((int)g_scratch.size() <= device) g_scratch.resize(device + 1, nullptr);
-    if (!g_scratch[device]) {
+    if ((int)g_scratch.size() <= *device) g_scratch.resize(*device + 1, nullptr);
+    cudaMemPool_t& pool = g_scratch[*device];
+    if (!pool) {
         cudaMemPoolProps props{};
         props.allocType = cudaMemAllocationTypePinned;
         props.location.type = cudaMemLocationTypeDevice;
-        props.location.id = device;
-        cudaMemPool_t pool = nullptr;
-        *err = cudaMemPoolCreate(&pool, &props);
-        if (*err != cudaSuccess) return nullptr;
+        props.location.id = *device;
+        cudaMemPool_t made = nullptr;
+        e = cudaMemPoolCreate(&made, &props);
+        if (e != cudaSuccess) return e;
         unsigned long long keep = kScratchKeep;
-        *err = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
-        if (*err != cudaSuccess) {
-            cudaMemPoolDestroy(pool);
-            return nullptr;
+        e = cudaMemPoolSetAttribute(made, cudaMemPoolAttrReleaseThreshold, &keep);
+        if (e != cudaSuccess) {
+            cudaMemPoolDestroy(made);
+            return e;
         }
-        g_scratch[device] = pool;
+        pool = made;
     }
-    return g_scratch[device];
+    *out = pool;
+    return cudaSuccess;
+}
+
+}  // namespace
+
+cudaError_t luz_scratch_alloc(void** p, size_t bytes, cudaStream_t st)
+{
+    cudaMemPool_t pool = nullptr;
+    int device = 0;
+    cudaError_t e = scratch_pool(&pool, &device);
+    if (e != cudaSuccess) return e;
+    e = cudaMallocFromPoolAsync(p, bytes, pool, st);
+    if (e == cudaErrorMemoryAllocation) {   // idle blocks of other sizes go back first
+        (void)cudaGetLastError();
+        luz_scratch_trim(device);
+        e = cudaMallocFromPoolAsync(p, bytes, pool, st);
+    }
+    return e;
 }
 
 void luz_scratch_trim(int device)
 {
     std::lock_guard<std::mutex> lock(g_scratch_mu);
-    if (device < 0 || device >= (int)g_scratch.size() || !g_scratch[device]) return;
-    cudaSetDevice(device);
-    cudaDeviceSynchronize();   // releases still in flight on a stream are not trimmed
-    cudaMemPoolTrimTo(g_scratch[device], 0);
+    if (device >= 0 && device < (int)g_scratch.size() && g_scratch[device]) cudaMemPoolTrimTo(g_scratch[device], 0);
 }
 
 struct luz_gpu_scene {
@@ -1264,7 +1291,6 @@ struct luz_gpu_scene {
             } catch (const Status& e) {
                 free_paths();
                 (void)cudaGetLastError();   // clears the allocation error
-                luz_scratch_trim(device);
                 if (e.code != LUZ_E_CUDA || n <= floor_n) throw;
                 n = std::max(floor_n, n / 2);
             }

@@ -616,24 +616,23 @@ struct NforError {
         if (e_ != cudaSuccess) throw NforError{LUZ_E_CUDA, std::string(#x) + ": " + cudaGetErrorString(e_)}; \
     } while (0)
 
-// Scratch arrays of one call, from the device's pool, in the order of stream st.
+// Scratch arrays of one call, from the device's pool, in the order of stream st; given back at
+// the end of the call, which waits for the stream.
 struct Buffers {
     cudaStream_t st;
     std::vector<void*> p;
     explicit Buffers(cudaStream_t s) : st(s) {}
     double* get(size_t n)
     {
-        cudaError_t e = cudaSuccess;
-        const cudaMemPool_t pool = luz_scratch_pool(&e);
-        NCK(e);
         void* q = nullptr;
-        NCK(cudaMallocFromPoolAsync(&q, sizeof(double) * (n ? n : 1), pool, st));
+        NCK(luz_scratch_alloc(&q, sizeof(double) * (n ? n : 1), st));
         p.push_back(q);
         return static_cast<double*>(q);
     }
     ~Buffers()
     {
         for (void* q : p) cudaFreeAsync(q, st);
+        cudaStreamSynchronize(st);
     }
 };
 

@@ -10,7 +10,7 @@
 
 // Denoise::applyNFOR (src/core/Denoise/NFOR.cpp:977-1102) on device-resident
 // NFOR buffers laid out as LuzNforBuffers; writes width*height*3 doubles to
-// d_out in `stream`'s order. settings NULL = NFORSettings defaults.
+// d_out and waits for `stream`. settings NULL = NFORSettings defaults.
 // Returns LUZ_OK, or a LUZ_E_* code with its message in msg.
 int luz_nfor_on_device(const double* color_a, const double* color_b, const double* color_variance,
                        const double* features_a, const double* features_b, const double* feature_variance,
@@ -21,12 +21,13 @@ int luz_nfor_on_device(const double* color_a, const double* color_b, const doubl
 // rows) comes from one stream-ordered pool per device instead of cudaMalloc: an allocation
 // and its release cost 0.6 ms there, and these calls make 3 to 45 of them. The pool keeps at
 // most kScratchKeep bytes between calls (what lies above goes back to the device at the next
-// synchronisation), gives all of it back when the last handle of the device is destroyed or
-// an allocation outside it fails, and orders reuse between streams and threads by the
-// streams' own dependencies.
+// synchronisation) and gives all of it back when the last handle of the device is destroyed
+// and when the device refuses this library an allocation, which is then tried again. Reuse
+// between streams and threads is ordered by the streams' own dependencies.
 constexpr unsigned long long kScratchKeep = 3ull << 30;
 
-// The current device's scratch pool; on failure NULL, with the CUDA error in *err.
-cudaMemPool_t luz_scratch_pool(cudaError_t* err);
-// Gives what the pool of `device` holds unused back to the device.
+// `bytes` from the current device's scratch pool in the order of `st` (cudaFreeAsync gives
+// them back; a call waits for its streams after that, so that what it gave back can be trimmed).
+cudaError_t luz_scratch_alloc(void** p, size_t bytes, cudaStream_t st);
+// Gives what the pool of `device` holds idle back to the device.
 void luz_scratch_trim(int device);

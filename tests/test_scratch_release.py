@@ -1,0 +1,44 @@
+"""What the scratch pool holds and when it lets go of it, each case in a process of its own."""
+import subprocess
+import sys
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+HEAD = """
+import sys
+import numpy as np, torch
+from luz_b200 import native, scenes
+sys.path.insert(0, 'tests')
+from test_scratch import buffers
+torch.cuda.init(); torch.zeros(1, device='cuda')
+free = lambda: torch.cuda.mem_get_info()[0]
+"""
+
+
+def run(code: str):
+    r = subprocess.run([sys.executable, "-c", HEAD + code], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
+def test_allocations_take_back_what_the_pool_holds_idle():
+    """With more than 1 GiB idle in the pool and all but 64 MiB of the device taken by others, a
+    scene of 131 MB, its first render (two 2^19-path waves' state) and a batch still find room."""
+    run("""
+w = scenes.mesh_glossy(256, 256, 8, 3, level=8)
+b = w.scene.build()
+small = scenes.mesh_glossy(64, 64, 1, 3, level=3)
+p, ps = (native.params(x.width, x.height, x.spp, 3, 5) for x in (w, small))
+g = native.GpuScene(b); want, _ = g.render(p); g.close()
+keep = native.GpuScene(small.scene.build())
+keep.render(ps); native.batch_render([keep], [ps])
+f0 = free()
+native.nfor_denoise(buffers(1280, 900, 1))
+idle = f0 - free()
+assert idle > 1 << 30, idle
+hog = torch.empty(max(0, free() - (64 << 20)), dtype=torch.uint8, device='cuda')
+g = native.GpuScene(b)
+film, st = g.render(p)
+assert np.array_equal(film, want) and st.waves == 1
+""")
