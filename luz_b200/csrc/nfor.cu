@@ -215,8 +215,13 @@ __device__ double patch_dist_at(const RegArgs& A, int x, int y, int sx, int sy)
 // terms (each with a FP64 division, which bounds it) per pixel and offset instead of a patch
 // of 9. The sums take the terms in patch order, so each distance has the same bits. Where the
 // neighbour itself is clamped to the image the terms are others: patch_dist_at. 960x540,
-// radius 2: 0.24 ms (0.55 with nine terms a thread); the filters' weights (radius 3) 0.53 ms
-// once, and 0.06 ms a filter that reads them (0.82 ms a filter that formed them).
+// radius 2: 0.24 ms (0.55 with nine terms a thread); the filters' weights (radius 3) 0.20 ms
+// once (0.53 with the whole window), and 0.06 ms a filter that reads them (0.82 ms a filter that formed them).
+//
+// WEIGHT stores half of the window: the weight of two pixels is the same from either (equal
+// terms in equal order), so row k of the first side * side / 2 serves both ways, and only
+// neighbours inside the image are stored: a clamped neighbour is one of them, at another offset
+// (filter_weight). 24 doubles a pixel instead of 49, no more than the regressions' distances.
 constexpr int kDistW = 32, kDistH = 8;
 constexpr int kDistTileMax = 48 * 1024;
 __host__ __device__ constexpr long long dist_tile_bytes(long long radius, long long patch)
@@ -242,7 +247,8 @@ __global__ void __launch_bounds__(kDistW* kDistH) k_patch_dist(RegArgs A, double
     const int lx = tid % kDistW, ly = tid / kDistW, x = x0 + lx, y = y0 + ly;
     const bool inside = x < I.w && y < I.h;
     const size_t npix = (size_t)I.w * I.h, pix = (size_t)y * I.w + x;
-    for (int k = 0; k < side * side; k++) {
+    const int K = WEIGHT ? side * side / 2 : side * side;
+    for (int k = 0; k < K; k++) {
         const int ox = k % side - R, oy = k / side - R;
         __syncthreads();   // the tile is loaded; the last offset's terms are read
         if (ox != 0 || oy != 0)
@@ -261,6 +267,8 @@ __global__ void __launch_bounds__(kDistW* kDistH) k_patch_dist(RegArgs A, double
                 for (int py = 0; py < pw; py++)
                     for (int px = 0; px < pw; px++) d += terms[(ly + py) * tcols + lx + px];
                 d = d / (double)(pw * pw);
+            } else if (WEIGHT) {
+                continue;
             } else {
                 d = patch_dist_at(A, x, y, clampc(x + ox, I.w), clampc(y + oy, I.h));
             }
@@ -543,6 +551,18 @@ __global__ void k_mse(Img I, const double* ca, const double* cb, const double* f
     mse2[i] = mse(fa2, fb2);
 }
 
+// The weight of pixel (x, y) and its clamped neighbour at offset (ox, oy), from the rows of
+// k_patch_dist<true> of that radius; s: the neighbour.
+__device__ __forceinline__ double filter_weight(Img I, const double* weight, int radius, int x, int y, int ox, int oy, int& s)
+{
+    const int sx = clampc(x + ox, I.w), sy = clampc(y + oy, I.h), side = 2 * radius + 1, half = side * side / 2;
+    const size_t npix = (size_t)I.w * I.h;
+    s = sy * I.w + sx;
+    const int k = (sy - y + radius) * side + (sx - x + radius);
+    if (k == half) return 1.0;   // the pixel itself: exp(-0)
+    return k < half ? weight[k * npix + (y * I.w + x)] : weight[(2 * half - k) * npix + s];
+}
+
 // filterScalarMapPair (NFOR.cpp:833-901): patch radius 1, bandwidth 1. select != 0
 // filters the bandwidth-selection maps of a and b instead of a and b. Both filters have the
 // same guide, hence the same weights: weight holds them (k_patch_dist<true>, as its rows).
@@ -555,12 +575,10 @@ __global__ void k_filter_pair(Img I, const double* a, const double* b, int selec
     auto vb = [&](int s) { return select ? (b[s] <= a[s] ? 1.0 : 0.0) : b[s]; };
     double fa = 0.0, fb = 0.0, total = 0.0;
     const int center = y * I.w + x;
-    const size_t npix = (size_t)I.w * I.h;
-    const double* w = weight + center;
     for (int oy = -radius; oy <= radius; oy++)
-        for (int ox = -radius; ox <= radius; ox++, w += npix) {
-            const int s = clampc(y + oy, I.h) * I.w + clampc(x + ox, I.w);
-            const double wgt = *w;
+        for (int ox = -radius; ox <= radius; ox++) {
+            int s;
+            const double wgt = filter_weight(I, weight, radius, x, y, ox, oy, s);
             fa += va(s) * wgt;
             fb += vb(s) * wgt;
             total += wgt;
@@ -672,8 +690,8 @@ void run_device(const double* ca, const double* cb, const double* cv, const doub
     double* rb2 = B.get(3 * n);
     const size_t K = (size_t)(2 * s.regression_radius + 1) * (2 * s.regression_radius + 1);
     constexpr int kFilterRadius = 3;
-    constexpr size_t kFilterWindow = (2 * kFilterRadius + 1) * (2 * kFilterRadius + 1);
-    double* dist = B.get((K > kFilterWindow ? K : kFilterWindow) * n);
+    constexpr size_t kFilterRows = (2 * kFilterRadius + 1) * (2 * kFilterRadius + 1) / 2;
+    double* dist = B.get((K > kFilterRows ? K : kFilterRows) * n);
     const dim3 dgrid((unsigned)((width + kDistW - 1) / kDistW), (unsigned)((height + kDistH - 1) / kDistH));
     // systems left to regression_half: at most two per pixel, 32 bits each; and their number
     unsigned* list = reinterpret_cast<unsigned*>(B.get(n));

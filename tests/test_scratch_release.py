@@ -42,3 +42,19 @@ g = native.GpuScene(b)
 film, st = g.render(p)
 assert np.array_equal(film, want) and st.waves == 1
 """)
+
+
+def test_the_denoiser_holds_133_doubles_a_pixel():
+    """Inputs and output 43, suppressed colours 9, prefiltered features 22, regressions 12, patch
+    distances 25, maps 6, blended colours, features and variance 15, list 1; the pool keeps what
+    a call took, below its bound of 3 GiB. Allowed beside that: 128 MiB of granularity."""
+    run("""
+w = scenes.mesh_glossy(8, 8, 1, 1, level=2)
+g = native.GpuScene(w.scene.build())
+native.nfor_denoise(buffers(8, 8, 1))
+f0 = free()
+n = 1600 * 900
+native.nfor_denoise(buffers(1600, 900, 2))
+held = f0 - free()
+assert held <= 133 * 8 * n + (128 << 20), (held, 133 * 8 * n)
+""")
