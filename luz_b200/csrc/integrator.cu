@@ -1060,20 +1060,6 @@ struct DeviceScratch {
     }
 };
 
-// Handles (scenes, caches) alive per device: the last one's end empties the scratch pool.
-std::mutex g_handles_mu;
-std::map<int, int> g_handles;
-void handle_opened(int device)
-{
-    std::lock_guard<std::mutex> lock(g_handles_mu);
-    g_handles[device]++;
-}
-void handle_closed(int device)
-{
-    std::lock_guard<std::mutex> lock(g_handles_mu);
-    if (--g_handles[device] == 0) luz_scratch_trim(device);
-}
-
 uint64_t next_scene_uid()
 {
     static std::atomic<uint64_t> n{0};
@@ -1095,6 +1081,8 @@ int guard(const std::function<int()>& f)
 
 std::mutex g_scratch_mu;
 std::vector<cudaMemPool_t> g_scratch;   // per device, created on first use, kept for the process
+std::mutex g_users_mu;
+std::map<int, int> g_users;             // handles and handle-less calls alive, per device
 
 }  // namespace
 
@@ -1145,6 +1133,18 @@ cudaError_t luz_scratch_alloc(void** p, size_t bytes, cudaStream_t st)
     return e;
 }
 
+void luz_scratch_open(int device)
+{
+    std::lock_guard<std::mutex> lock(g_users_mu);
+    g_users[device]++;
+}
+
+void luz_scratch_close(int device)
+{
+    std::lock_guard<std::mutex> lock(g_users_mu);
+    if (--g_users[device] == 0) luz_scratch_trim(device);
+}
+
 void luz_scratch_trim(int device)
 {
     std::lock_guard<std::mutex> lock(g_scratch_mu);
@@ -1153,7 +1153,7 @@ void luz_scratch_trim(int device)
 
 struct luz_gpu_scene {
     int device = 0;
-    bool counted = false;            // among the device's live handles
+    bool counted = false;            // among the users of the device's scratch pool
     std::unique_ptr<ScenePack> pack;
     DScene ds{};
     DScene* dds = nullptr;           // device copy of ds: k_shade reads it through a pointer so that
@@ -1317,7 +1317,7 @@ struct luz_gpu_scene {
         for (cudaEvent_t e : {lane_setup, lane_done, lane_acc[0], lane_acc[1]})
             if (e) cudaEventDestroy(e);
         if (stream2) cudaStreamDestroy(stream2);
-        if (counted) handle_closed(device);
+        if (counted) luz_scratch_close(device);
     }
     void ensure_lanes()
     {
@@ -2957,7 +2957,7 @@ int luz_gpu_scene_create(const LuzSceneDesc* desc, int32_t device, luz_gpu_scene
         s->pack.reset(pack_scene(desc));
         s->device = device;
         CK(cudaSetDevice(device));
-        handle_opened(device);
+        luz_scratch_open(device);
         s->counted = true;
         CK(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking));
         CK(cudaEventCreate(&s->ev0));
@@ -3429,7 +3429,7 @@ struct luz_gpu_cache {
         cudaSetDevice(device);
         for (void* p : {(void*)W, (void*)G, (void*)m, (void*)v, (void*)loss, (void*)Wf, (void*)Wb})
             if (p) cudaFree(p);
-        if (counted) handle_closed(device);
+        if (counted) luz_scratch_close(device);
     }
 };
 
@@ -3639,7 +3639,7 @@ int luz_gpu_cache_create(int32_t device, const LuzCacheParams* prm, luz_gpu_cach
         CK(cudaSetDevice(device));
         std::unique_ptr<luz_gpu_cache> c(new luz_gpu_cache);
         c->device = device;
-        handle_opened(device);
+        luz_scratch_open(device);
         c->counted = true;
         c->prm = *prm;
         c->W = dalloc<float>(kCacheParams);

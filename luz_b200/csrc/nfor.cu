@@ -14,8 +14,10 @@
 // the last bit.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <initializer_list>
 #include <string>
 #include <vector>
 
@@ -647,11 +649,28 @@ struct Buffers {
         p.push_back(q);
         return static_cast<double*>(q);
     }
+    // Arrays no later kernel reads go back for the next ones to take (others than its own stay).
+    void drop(std::initializer_list<const double*> done)
+    {
+        for (const double* d : done) {
+            const auto i = std::find(p.begin(), p.end(), static_cast<const void*>(d));
+            if (i == p.end()) continue;
+            cudaFreeAsync(*i, st);
+            p.erase(i);
+        }
+    }
     ~Buffers()
     {
         for (void* q : p) cudaFreeAsync(q, st);
         cudaStreamSynchronize(st);
     }
+};
+
+// A denoise on its way as a user of the device's scratch pool.
+struct PoolUser {
+    int device;
+    explicit PoolUser(int d) : device(d) { luz_scratch_open(d); }
+    ~PoolUser() { luz_scratch_close(device); }
 };
 
 LuzNforSettings checked_settings(const LuzNforSettings* st)
@@ -663,9 +682,10 @@ LuzNforSettings checked_settings(const LuzNforSettings* st)
     return s;
 }
 
+// in: the owner of the inputs that may go as soon as they are read, NULL when they stay.
 void run_device(const double* ca, const double* cb, const double* cv, const double* ga, const double* gb,
                 const double* gv, int32_t width, int32_t height, const LuzNforSettings& s, double* d_out,
-                cudaStream_t st)
+                cudaStream_t st, Buffers* in)
 {
     const size_t n = (size_t)width * height;
     Buffers B(st);
@@ -678,11 +698,13 @@ void run_device(const double* ca, const double* cb, const double* cv, const doub
     k_firefly<<<grd, blk, 0, st>>>(I, ca, nullptr, fa);
     k_firefly<<<grd, blk, 0, st>>>(I, cb, nullptr, fb);
     k_firefly<<<grd, blk, 0, st>>>(I, fa, fb, col);
+    if (in) in->drop({ca, cb});
     // features prefiltered with the other half as the guide
     double* pfa = B.get(kF * n);
     double* pfb = B.get(kF * n);
     k_prefilter<<<grd, blk, 0, st>>>(I, ga, gb, gv, s.feature_prefilter_radius, s.min_variance, pfa);
     k_prefilter<<<grd, blk, 0, st>>>(I, gb, ga, gv, s.feature_prefilter_radius, s.min_variance, pfb);
+    if (in) in->drop({ga, gb, gv});
     // two-bandwidth regressions (variance doubled)
     double* ra1 = B.get(3 * n);
     double* ra2 = B.get(3 * n);
@@ -722,18 +744,22 @@ void run_device(const double* ca, const double* cb, const double* cv, const doub
     double* m2 = B.get(n);
     double* fm1 = B.get(n);
     double* fm2 = B.get(n);
-    double* s1 = B.get(n);
-    double* s2 = B.get(n);
     k_mse<<<grd, blk, 0, st>>>(I, fa, fb, ra1, rb1, ra2, rb2, cv, m1, m2);
+    B.drop({fa, fb});
     const RegArgs W{I, col, nullptr, cv, 1.0, kFilterRadius, 1, s.min_variance, 1.0, -1.0, nullptr, nullptr, nullptr};
     k_patch_dist<true><<<dgrid, kDistW * kDistH, (size_t)dist_tile_bytes(kFilterRadius, 1), st>>>(W, dist);
+    B.drop({col});
     k_filter_pair<<<grd, blk, 0, st>>>(I, m1, m2, 0, dist, kFilterRadius, fm1, fm2);
+    B.drop({m1, m2});
+    double* s1 = B.get(n);
+    double* s2 = B.get(n);
     k_filter_pair<<<grd, blk, 0, st>>>(I, fm1, fm2, 1, dist, kFilterRadius, s1, s2);
     // blend, final features and variance, last regression
     double* comb = B.get(3 * n);
     double* ff = B.get(kF * n);
     double* fv = B.get(n);
     k_combine<<<grd, blk, 0, st>>>(I, s1, s2, fm1, fm2, ra1, ra2, rb1, rb2, pfa, pfb, s.min_variance, comb, ff, fv);
+    B.drop({pfa, pfb, ra1, ra2, rb1, rb2, fm1, fm2, s1, s2});
     RegArgs C{I, comb, ff, fv, 1.0, s.regression_radius, s.patch_radius, s.min_variance, 1.0, -1.0, d_out, nullptr, dist};
     regress(C);
     NCK(cudaGetLastError());
@@ -750,6 +776,7 @@ int do_nfor(int32_t device, const LuzNforBuffers* in, int32_t width, int32_t hei
         throw NforError{LUZ_E_INVALID, "NFOR needs every buffer."};
     NCK(cudaSetDevice(device));
     const size_t n = (size_t)width * height;
+    PoolUser user(device);   // goes after the buffers: without a handle open the device gets them back
     Buffers B(0);
     double* ca = B.get(3 * n);
     double* cb = B.get(3 * n);
@@ -764,7 +791,7 @@ int do_nfor(int32_t device, const LuzNforBuffers* in, int32_t width, int32_t hei
     NCK(cudaMemcpy(ga, in->features_a, sizeof(double) * kF * n, cudaMemcpyHostToDevice));
     NCK(cudaMemcpy(gb, in->features_b, sizeof(double) * kF * n, cudaMemcpyHostToDevice));
     NCK(cudaMemcpy(gv, in->feature_variance, sizeof(double) * kF * n, cudaMemcpyHostToDevice));
-    run_device(ca, cb, cv, ga, gb, gv, width, height, s, out, 0);
+    run_device(ca, cb, cv, ga, gb, gv, width, height, s, out, 0, &B);
     NCK(cudaMemcpy(rgb_out, out, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost));
     return LUZ_OK;
 }
@@ -778,7 +805,7 @@ int luz_nfor_on_device(const double* ca, const double* cb, const double* cv, con
     try {
         const LuzNforSettings s = checked_settings(settings);
         if (width > 0 && height > 0)
-            run_device(ca, cb, cv, ga, gb, gv, width, height, s, d_out, (cudaStream_t)stream);
+            run_device(ca, cb, cv, ga, gb, gv, width, height, s, d_out, (cudaStream_t)stream, nullptr);
         return LUZ_OK;
     } catch (const NforError& e) {
         msg = e.msg;

@@ -21,13 +21,17 @@ int luz_nfor_on_device(const double* color_a, const double* color_b, const doubl
 // rows) comes from one stream-ordered pool per device instead of cudaMalloc: an allocation
 // and its release cost 0.6 ms there, and these calls make 3 to 45 of them. The pool keeps at
 // most kScratchKeep bytes between calls (what lies above goes back to the device at the next
-// synchronisation) and gives all of it back when the last handle of the device is destroyed
-// and when the device refuses this library an allocation, which is then tried again. Reuse
-// between streams and threads is ordered by the streams' own dependencies.
+// synchronisation) and gives all of it back when the last user of the device goes (a scene or
+// cache handle, or a denoise under way without one) and when the device refuses this library
+// an allocation, which is then tried again. Reuse between streams and threads is ordered by the
+// streams' own dependencies.
 constexpr unsigned long long kScratchKeep = 3ull << 30;
 
 // `bytes` from the current device's scratch pool in the order of `st` (cudaFreeAsync gives
 // them back; a call waits for its streams after that, so that what it gave back can be trimmed).
 cudaError_t luz_scratch_alloc(void** p, size_t bytes, cudaStream_t st);
+// A user of the pool of `device` comes and goes; the last one's leaving empties the pool.
+void luz_scratch_open(int device);
+void luz_scratch_close(int device);
 // Gives what the pool of `device` holds idle back to the device.
 void luz_scratch_trim(int device);

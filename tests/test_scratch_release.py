@@ -22,6 +22,20 @@ def run(code: str):
     assert r.returncode == 0, r.stdout + r.stderr
 
 
+def test_a_denoise_without_handles_keeps_nothing():
+    """No scene or cache is ever opened: after a denoise the device holds what it held after a
+    denoise of 8 x 8 pixels, which loads the same kernels (to 32 MiB; the 960 x 540 buffers are
+    more than ten times that)."""
+    run("""
+native.nfor_denoise(buffers(8, 8, 1))
+free0 = free()
+for k in range(3):
+    native.nfor_denoise(buffers(960, 540, k))
+left = free0 - free()
+assert left <= 32 << 20, left
+""")
+
+
 def test_allocations_take_back_what_the_pool_holds_idle():
     """With more than 1 GiB idle in the pool and all but 64 MiB of the device taken by others, a
     scene of 131 MB, its first render (two 2^19-path waves' state) and a batch still find room."""
@@ -34,7 +48,7 @@ g = native.GpuScene(b); want, _ = g.render(p); g.close()
 keep = native.GpuScene(small.scene.build())
 keep.render(ps); native.batch_render([keep], [ps])
 f0 = free()
-native.nfor_denoise(buffers(1280, 900, 1))
+native.nfor_denoise(buffers(1920, 1080, 1))
 idle = f0 - free()
 assert idle > 1 << 30, idle
 hog = torch.empty(max(0, free() - (64 << 20)), dtype=torch.uint8, device='cuda')
