@@ -109,6 +109,7 @@ __host__ __device__ constexpr int progressive_place(uint32_t dim)
 }
 constexpr int kProgressiveDims = 7;
 constexpr int kStepBounces = 256;   // bounces the step table covers (every render's: kMaxBounceSlots)
+static_assert((kStepBounces & (kStepBounces - 1)) == 0, "dim_step masks the bounce");
 
 // Lattice step of the dimension key dk = dim + bounce * 32 and the component: a function of
 // those two alone.

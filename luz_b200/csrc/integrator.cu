@@ -55,6 +55,8 @@ __global__ void __launch_bounds__(kBlock) k_raygen(WaveArgs w, PathBuf P, Ctrl* 
 
 // ---------------------------------------------------------------------------- trace (closest and any hits)
 
+static_assert(kBlock == kWalkBlock, "WorldRays holds a ray per thread of a trace block");
+
 // Resident blocks per SM the register allocator is asked to allow, measured on one B200:
 // 8 blocks (64 registers) 214.8 ms on the 1080p glossy frame at 64 spp, 7 (72) 223.5, 9 (56)
 // 217.8, 10 224.7; with instances 6 (80) 203.7 ms on the 1e5-instance frame at 8 spp, 5 213.9,
@@ -3404,7 +3406,7 @@ int luz_gpu_trace_rays(luz_gpu_scene* s, const float* rays, int64_t count, int32
         clear_error(s, st);
         CK(cudaMemcpyAsync(dr, rays, sizeof(float) * 8 * count, cudaMemcpyHostToDevice, st));
         if (dk) CK(cudaMemcpyAsync(dk, volume_key, sizeof(int32_t) * 4 * count, cudaMemcpyHostToDevice, st));
-        kTraceRayKernels[s->ds.k.features & TF_ALL]<<<(unsigned)((count + 127) / 128), 128, 0, st>>>(
+        kTraceRayKernels[s->ds.k.features & TF_ALL]<<<(unsigned)((count + kWalkBlock - 1) / kWalkBlock), kWalkBlock, 0, st>>>(
             s->ds, dr, count, any_hit, seed, dk, dh);
         CK(cudaGetLastError());
         CK(cudaMemcpyAsync(out, dh, sizeof(LuzHit) * count, cudaMemcpyDeviceToHost, st));

@@ -434,6 +434,7 @@ __device__ void regression_half(const RegArgs& A, long long pix, bool second)
 // one half 1.63 ms (6.68 with regression_half for every pixel), the last regression 0.91 ms
 // (3.35); against that solver the image moves by 1e-15.
 constexpr int kRegWarps = 8;
+constexpr int kRestBlocks = 148;         // of the systems left over: one per SM, each takes a share of the list
 constexpr int kRegTileMax = 48 * 1024;   // shared memory of a tile: up to radius 6 (pairs), 4 (single)
 __host__ __device__ constexpr int reg_pixels(bool pair) { return kRegWarps * (pair ? 2 : 4); }
 __host__ __device__ constexpr long long reg_tile_bytes(bool pair, long long radius)
@@ -733,7 +734,7 @@ void run_device(const double* ca, const double* cb, const double* cv, const doub
         const dim3 grid((unsigned)((width + reg_pixels(pair) - 1) / reg_pixels(pair)), (unsigned)height);
         if (pair) k_regression<true><<<grid, 32 * kRegWarps, (size_t)tile, st>>>(A, list, list_n);
         else k_regression<false><<<grid, 32 * kRegWarps, (size_t)tile, st>>>(A, list, list_n);
-        k_regression_warp<<<148, 128, 0, st>>>(A, list, list_n);
+        k_regression_warp<<<kRestBlocks, 128, 0, st>>>(A, list, list_n);
     };
     RegArgs A{I, fa, pfb, cv, 2.0, s.regression_radius, s.patch_radius, s.min_variance, 0.5, 1.0, ra1, ra2, dist};
     regress(A);

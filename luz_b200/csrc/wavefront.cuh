@@ -8,8 +8,10 @@
 namespace luz {
 
 constexpr int kMaxBounceSlots = 256;
+static_assert(kMaxBounceSlots <= kStepBounces, "every bounce has its lattice steps in the table");
 constexpr int kBlock = 128;
 constexpr int kShadeClasses = 10;           // 0 = miss, 1..9 = material type of the hit
+static_assert(MT_DIFFUSE_GLOSSY < kShadeClasses, "a class per material type");
 
 struct Ctrl {
     uint32_t count[kMaxBounceSlots + 2];    // extension queue size entering bounce b
