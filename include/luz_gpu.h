@@ -248,7 +248,8 @@ typedef struct LuzRenderStats {
     int64_t  kernel_launches;     /* kernels launched by this call                  */
     int64_t  waves;
     double   extend_ms, shade_ms, shadow_ms;   /* LUZ_RENDER_PROFILE: summed stage times */
-    int64_t  extend_launches, shadow_launches;
+    int64_t  extend_launches, shadow_launches; /* launches that hold closest-hit / any-hit rays (a  */
+                                               /* launch holds both unless LUZ_RENDER_PROFILE set)  */
     double   ext_nodes, ext_tris, ext_top;     /* LUZ_RENDER_COUNT: mesh nodes, triangles,  */
     double   sh_nodes, sh_tris, sh_top;        /* top-level records read (ext / shadow)     */
     double   denoise_ms;          /* luz_gpu_render_denoised: device time of NFOR    */

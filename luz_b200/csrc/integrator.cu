@@ -165,7 +165,7 @@ __device__ __forceinline__ void trace_extension(const DScene& S, const WaveArgs&
             const THit h = walk.h;
             P.hit[p] = make_float4(h.t, h.u, h.v, __int_as_float(h.obj));
             P.hit_prim[p] = h.prim;
-            if (P.bins) bin_append(C->bin[bounce], P, vmask, h.obj < 0 ? 0u : (uint32_t)S.obj_class[h.obj], p);
+            bin_append(C->bin[bounce], P, vmask, h.obj < 0 ? 0u : (uint32_t)S.obj_class[h.obj], p);
             if constexpr (COUNT) {
                 atomicAdd(&S.counters[0], (unsigned long long)walk.n_nodes);
                 atomicAdd(&S.counters[1], (unsigned long long)walk.n_tris);
@@ -2357,7 +2357,7 @@ int do_adjoint_density(luz_gpu_scene* s, const LuzRenderParams* p, int32_t objec
 // arrays in one allocation, reused while the same scene contents come back), the
 // table of DScene records pointing into it, the shared path state, the segment
 // tables and the CUDA graph of one wave. A wave is recorded once per batch call
-// (raygen, every bounce's extend / shade / shadow, accumulate) and replayed for
+// (raygen, every bounce's trace and shade, the last shadow rays, accumulate) and replayed for
 // every wave with that wave's segment table copied to a fixed device address.
 
 constexpr int64_t kBatchWaveDefault = int64_t(1) << 24;

@@ -1556,7 +1556,7 @@ ScenePack* pack_scene(const LuzSceneDesc* d)
             E.pdf_offset = -1;
         }
     }
-    // Shade binning: the material type (1..7) a hit on each object shades with
+    // Shade binning: the material type (1..9) a hit on each object shades with
     // (make_hit: a mesh shades with its mesh's material, every other kind with its own).
     S.obj_class.assign(S.objects.size(), 0);
     for (std::size_t i = 0; i < S.objects.size(); i++) {
