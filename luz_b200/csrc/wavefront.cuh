@@ -743,7 +743,12 @@ static __device__ void shade_path(const DScene& S, const WaveArgs& w, const Path
         }
         if (MODE == 3 && w.adjoint && w.grad_kind == 0 && m.type == MT_LAMBERTIAN && m.texture == w.grad_texture) {
             if (w.adj_vertices) {
-                const unsigned long long i = atomicAdd(w.adj_count, 1ull);
+                // one atomic for the lanes that are here together
+                const unsigned here = __activemask();
+                const int first = __ffs(here) - 1;
+                unsigned long long i = 0;
+                if ((int)lane_id() == first) i = atomicAdd(w.adj_count, (unsigned long long)__popc(here));
+                i = __shfl_sync(here, i, first) + (unsigned)__popc(here & ((1u << lane_id()) - 1u));
                 if (i < w.adj_cap) w.adj_vertices[i] = AdjVertex{{rad.x, rad.y, rad.z}, h.u, h.v, p};
             } else {
                 const float4 L = P.color[p];
