@@ -150,7 +150,8 @@ def profile_counters():
     """Per-extension-ray ncu figures of k_trace from the committed summary: DRAM bytes,
     L2 bytes (lts__t_bytes), L2 throughput as a fraction of its peak
     (lts__throughput.avg.pct_of_peak_sustained_elapsed / 100) and active lanes per
-    warp instruction (smsp__thread_inst_executed_per_inst_executed)."""
+    warp instruction (smsp__thread_inst_executed_per_inst_executed) and the fraction of
+    issue slots used (smsp__issue_active / 100)."""
     import re
     out = {}
     if os.path.exists(PROFILE_SUMMARY):
@@ -158,7 +159,8 @@ def profile_counters():
         for key, pat in (("dram", r"DRAM bytes per extension ray: ([0-9.]+)"),
                          ("l2", r"L2 bytes per extension ray: ([0-9.]+)"),
                          ("l2_frac", r"L2 throughput, fraction of peak: ([0-9.]+)"),
-                         ("lanes", r"active lanes per warp instruction: ([0-9.]+)")):
+                         ("lanes", r"active lanes per warp instruction: ([0-9.]+)"),
+                         ("issue", r"issue slots used, fraction: ([0-9.]+)")):
             m = re.search(pat, txt)
             if m:
                 out[key] = float(m.group(1))
@@ -323,7 +325,10 @@ def run_ours(args):
         dist.all_reduce(t, op=dist.ReduceOp.MAX)
         e2 = float(t.item())
 
-    # roofline of the dominant kernel (closest-hit traversal), from an instrumented extra frame
+    # roofline of the dominant kernel (closest-hit traversal), from an instrumented extra frame.
+    # It is bound by instruction issue; the bytes of the binary walk that the collapsed one stands
+    # for come from L1 and L2, so their rate (walk_gbs) is a speed of the walk and no fraction of
+    # the memory's, whose own traffic stands beside it.
     pp = native.params(w.width, w.height, w.spp, w.max_bounces, w.seed, 0, rank * w.spp)
     pp.flags = RENDER_PROFILE | RENDER_COUNT
     prof = g.render_device(pp, film.data_ptr(), stream.cuda_stream)
@@ -339,10 +344,11 @@ def run_ours(args):
     launch_ms = timed.extend_ms / max(1, timed.extend_launches)
     rays_per_launch = ext_rays / max(1, prof.extend_launches)
     bytes_per_launch = alg_bytes / max(1, prof.extend_launches)
-    achieved = bytes_per_launch / (launch_ms * 1e-3) / 1e9 if launch_ms > 0 else None
+    walk_gbs = bytes_per_launch / (launch_ms * 1e-3) / 1e9 if launch_ms > 0 else None
     peak, peak_kind = measured_peak()
     pc = profile_counters()
     traffic = pc["dram"] * rays_per_launch if "dram" in pc else None
+    hbm_gbs = traffic / (launch_ms * 1e-3) / 1e9 if traffic and launch_ms > 0 else None
     l2_gbs = pc["l2"] * rays_per_launch / (launch_ms * 1e-3) / 1e9 if ("l2" in pc and launch_ms > 0) else None
 
     # the drop-in per frame as a host glue would run it: scene description, luz_gpu_scene_create
@@ -375,14 +381,18 @@ def run_ours(args):
                        "host_film": "pinned"},
                "gpu_launches": int(launches),
                "clocks": clk,
-               "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                            "frac": (achieved / peak) if achieved else None, "traffic": traffic,
-                            "kernel": "k_trace (closest-hit traversal, launched alone)", "peak_kind": peak_kind,
+               "roofline": {"bound": "issue", "achieved": pc.get("issue"), "peak": 1.0, "unit": "issue slots used",
+                            "frac": pc.get("issue"),
+                            "source": "ncu smsp__issue_active of a bounce-2 launch (profiles/k_trace_counters_mesh_glossy.md)",
+                            "kernel": "k_trace (closest-hit traversal, launched alone)",
+                            "rays_per_launch": rays_per_launch, "launch_ms": launch_ms,
+                            "grays_per_s": rays_per_launch / (launch_ms * 1e6) if launch_ms > 0 else None,
                             "algorithmic_bytes_per_ray": alg_bytes / max(1.0, ext_rays),
                             "bytes_formula": "64 x binary node visits + 48 x triangle tests + 32 x top-level "
                                              "records + 52 per ray",
-                            "rays_per_launch": rays_per_launch,
-                            "launch_ms": launch_ms,
+                            "walk_gbs": walk_gbs,
+                            "traffic": traffic, "hbm_gbs": hbm_gbs, "hbm_peak": peak, "hbm_peak_kind": peak_kind,
+                            "hbm_frac": hbm_gbs / peak if hbm_gbs else None,
                             "traffic_source": "ncu dram bytes per extension ray x rays per launch "
                                               "(profiles/k_trace_counters_mesh_glossy.md)",
                             "l2_gbs": l2_gbs, "l2_frac": pc.get("l2_frac"),

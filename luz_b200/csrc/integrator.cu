@@ -67,6 +67,8 @@ static_assert(kBlock == kWalkBlock, "WorldRays holds a ray per thread of a trace
 #ifndef LUZ_TRACE_MIN_BLOCKS_INST
 #define LUZ_TRACE_MIN_BLOCKS_INST 6
 #endif
+// Batches (always the code for instances and volumes): a batch of 12 small scenes takes 6.9 ms
+// at 6 blocks, 7.0-7.2 at 5, 7.0 at 8 and 7.8 at 10.
 #ifndef LUZ_TRACE_MIN_BLOCKS_BATCH
 #define LUZ_TRACE_MIN_BLOCKS_BATCH 6
 #endif
