@@ -465,7 +465,7 @@ def run_batch(args):
 def run_adjoint(args):
     """--workload adjoint_c3: albedo-texture gradient of the textured Cornell box (256x256,
     64 spp, depth 8, 32x32 back-wall texture): Madjoint paths/s = W*H*spp paths replayed per
-    second of luz_gpu_adjoint_backward (both passes), device time from the call's CUDA events;
+    second of luz_gpu_adjoint_backward, device time from the call's CUDA events;
     beside it the same figure for the 64x64 roughness map of a Metal panel in the box and for
     the light-emission gradient (luz_gpu_adjoint_emission)."""
     from luz_b200 import native, scenes

@@ -38,7 +38,7 @@ assert left <= 32 << 20, left
 
 def test_allocations_take_back_what_the_pool_holds_idle():
     """With more than 1 GiB idle in the pool and all but 64 MiB of the device taken by others, a
-    scene of 131 MB, its first render (two 2^19-path waves' state) and a batch still find room."""
+    scene of 131 MB and its first render (one wave of 2^19 paths, 145 MB of state) find room."""
     run("""
 w = scenes.mesh_glossy(256, 256, 8, 3, level=8)
 b = w.scene.build()
@@ -59,9 +59,10 @@ assert np.array_equal(film, want) and st.waves == 1
 
 
 def test_the_denoiser_holds_133_doubles_a_pixel():
-    """Inputs and output 43, suppressed colours 9, prefiltered features 22, regressions 12, patch
-    distances 25, maps 6, blended colours, features and variance 15, list 1; the pool keeps what
-    a call took, below its bound of 3 GiB. Allowed beside that: 128 MiB of granularity."""
+    """At most, were all of a call's arrays alive at once: inputs and output 43, suppressed colours
+    9, prefiltered features 22, regressions 12, patch distances 25, maps 6, blended colours,
+    features and variance 15, list 1. The pool keeps what a call took, below its bound of 3 GiB.
+    Allowed beside that: 128 MiB of granularity."""
     run("""
 w = scenes.mesh_glossy(8, 8, 1, 1, level=2)
 g = native.GpuScene(w.scene.build())
