@@ -1037,15 +1037,16 @@ template <class T> T* dupload(const std::vector<T>& v)
 }
 
 // Device buffers of one call, from the device's scratch pool in the order of their stream,
-// given back to it on every exit path; the call then waits for its stream (3 us: its work is
-// done), so that what the pool holds of it is idle and can be trimmed.
+// given back to it on every exit path. own_wait: see luz_scratch_alloc.
 struct DeviceScratch {
     std::vector<std::pair<void*, cudaStream_t>> ptrs;
+    const bool own_wait;
+    explicit DeviceScratch(bool own_wait_ = false) : own_wait(own_wait_) {}
     // n elements, not initialised
     template <class T> T* raw(int64_t n, cudaStream_t st)
     {
         void* p = nullptr;
-        CK(luz_scratch_alloc(&p, sizeof(T) * (std::size_t)std::max<int64_t>(n, 1), st));
+        CK(luz_scratch_alloc(&p, sizeof(T) * (std::size_t)std::max<int64_t>(n, 1), st, own_wait));
         ptrs.push_back({p, st});
         return static_cast<T*>(p);
     }
@@ -1059,7 +1060,7 @@ struct DeviceScratch {
     ~DeviceScratch()
     {
         for (auto& p : ptrs) cudaFreeAsync(p.first, p.second);
-        for (std::size_t i = 0; i < ptrs.size(); i++)
+        for (std::size_t i = 0; own_wait && i < ptrs.size(); i++)
             if (i == 0 || ptrs[i].second != ptrs[i - 1].second) cudaStreamSynchronize(ptrs[i].second);
     }
 };
@@ -1083,8 +1084,14 @@ int guard(const std::function<int()>& f)
     }
 }
 
+// Per device: the pool, created on first use and kept for the process, and the streams alive
+// that took from it.
+struct ScratchPool {
+    cudaMemPool_t pool = nullptr;
+    std::vector<cudaStream_t> streams;
+};
 std::mutex g_scratch_mu;
-std::vector<cudaMemPool_t> g_scratch;   // per device, created on first use, kept for the process
+std::vector<ScratchPool> g_scratch;
 std::mutex g_users_mu;
 std::map<int, int> g_users;             // handles and handle-less calls alive, per device
 
@@ -1092,14 +1099,14 @@ std::map<int, int> g_users;             // handles and handle-less calls alive, 
 
 namespace {
 
-// The current device's scratch pool.
-cudaError_t scratch_pool(cudaMemPool_t* out, int* device)
+// The current device's scratch pool, from which `st` is about to take (NULL st: not noted).
+cudaError_t scratch_pool(cudaMemPool_t* out, int* device, const cudaStream_t* st)
 {
     cudaError_t e = cudaGetDevice(device);
     if (e != cudaSuccess) return e;
     std::lock_guard<std::mutex> lock(g_scratch_mu);
-    if ((int)g_scratch.size() <= *device) g_scratch.resize(*device + 1, nullptr);
-    cudaMemPool_t& pool = g_scratch[*device];
+    if ((int)g_scratch.size() <= *device) g_scratch.resize(*device + 1);
+    cudaMemPool_t& pool = g_scratch[*device].pool;
     if (!pool) {
         cudaMemPoolProps props{};
         props.allocType = cudaMemAllocationTypePinned;
@@ -1116,17 +1123,19 @@ cudaError_t scratch_pool(cudaMemPool_t* out, int* device)
         }
         pool = made;
     }
+    std::vector<cudaStream_t>& streams = g_scratch[*device].streams;
+    if (st && std::find(streams.begin(), streams.end(), *st) == streams.end()) streams.push_back(*st);
     *out = pool;
     return cudaSuccess;
 }
 
 }  // namespace
 
-cudaError_t luz_scratch_alloc(void** p, size_t bytes, cudaStream_t st)
+cudaError_t luz_scratch_alloc(void** p, size_t bytes, cudaStream_t st, bool own_wait)
 {
     cudaMemPool_t pool = nullptr;
     int device = 0;
-    cudaError_t e = scratch_pool(&pool, &device);
+    cudaError_t e = scratch_pool(&pool, &device, own_wait ? nullptr : &st);
     if (e != cudaSuccess) return e;
     e = cudaMallocFromPoolAsync(p, bytes, pool, st);
     if (e == cudaErrorMemoryAllocation) {   // idle blocks of other sizes go back first
@@ -1152,7 +1161,20 @@ void luz_scratch_close(int device)
 void luz_scratch_trim(int device)
 {
     std::lock_guard<std::mutex> lock(g_scratch_mu);
-    if (device >= 0 && device < (int)g_scratch.size() && g_scratch[device]) cudaMemPoolTrimTo(g_scratch[device], 0);
+    if (device < 0 || device >= (int)g_scratch.size() || !g_scratch[device].pool) return;
+    for (cudaStream_t st : g_scratch[device].streams) cudaStreamSynchronize(st);
+    cudaMemPoolTrimTo(g_scratch[device].pool, 0);
+}
+
+void luz_scratch_forget(int device, cudaStream_t st)
+{
+    std::lock_guard<std::mutex> lock(g_scratch_mu);
+    if (device < 0 || device >= (int)g_scratch.size()) return;
+    std::vector<cudaStream_t>& streams = g_scratch[device].streams;
+    const auto i = std::find(streams.begin(), streams.end(), st);
+    if (i == streams.end()) return;
+    cudaStreamSynchronize(st);
+    streams.erase(i);
 }
 
 struct luz_gpu_scene {
@@ -1316,7 +1338,10 @@ struct luz_gpu_scene {
         if (totals) cudaFree(totals);
         if (ev0) cudaEventDestroy(ev0);
         if (ev1) cudaEventDestroy(ev1);
-        if (stream) cudaStreamDestroy(stream);
+        if (stream) {
+            luz_scratch_forget(device, stream);
+            cudaStreamDestroy(stream);
+        }
         if (ctrl2) cudaFree(ctrl2);
         for (cudaEvent_t e : {lane_setup, lane_done, lane_acc[0], lane_acc[1]})
             if (e) cudaEventDestroy(e);
@@ -2640,7 +2665,7 @@ int batch_render(luz_gpu_scene* const* scenes, const LuzRenderParams* params, in
         film_doubles += 3 * npix;
         out_floats += 3 * npix;
     }
-    DeviceScratch D;
+    DeviceScratch D(true);   // C.st captures the wave's graph
     double* films = D.get<double>(film_doubles, st);
     float* outs = D.get<float>(out_floats, st);
     double** d_films = D.get<double*>(count, st);

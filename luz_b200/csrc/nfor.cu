@@ -637,8 +637,7 @@ struct NforError {
         if (e_ != cudaSuccess) throw NforError{LUZ_E_CUDA, std::string(#x) + ": " + cudaGetErrorString(e_)}; \
     } while (0)
 
-// Scratch arrays of one call, from the device's pool, in the order of stream st; given back at
-// the end of the call, which waits for the stream.
+// Scratch arrays of one call, from the device's pool, in the order of stream st.
 struct Buffers {
     cudaStream_t st;
     std::vector<void*> p;
@@ -663,7 +662,6 @@ struct Buffers {
     ~Buffers()
     {
         for (void* q : p) cudaFreeAsync(q, st);
-        cudaStreamSynchronize(st);
     }
 };
 

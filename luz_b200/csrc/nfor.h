@@ -10,7 +10,7 @@
 
 // Denoise::applyNFOR (src/core/Denoise/NFOR.cpp:977-1102) on device-resident
 // NFOR buffers laid out as LuzNforBuffers; writes width*height*3 doubles to
-// d_out and waits for `stream`. settings NULL = NFORSettings defaults.
+// d_out in `stream`'s order. settings NULL = NFORSettings defaults.
 // Returns LUZ_OK, or a LUZ_E_* code with its message in msg.
 int luz_nfor_on_device(const double* color_a, const double* color_b, const double* color_variance,
                        const double* features_a, const double* features_b, const double* feature_variance,
@@ -27,9 +27,14 @@ int luz_nfor_on_device(const double* color_a, const double* color_b, const doubl
 // streams' own dependencies.
 constexpr unsigned long long kScratchKeep = 3ull << 30;
 
-// `bytes` from the current device's scratch pool in the order of `st` (cudaFreeAsync gives
-// them back; a call waits for its streams after that, so that what it gave back can be trimmed).
-cudaError_t luz_scratch_alloc(void** p, size_t bytes, cudaStream_t st);
+// `bytes` from the current device's scratch pool in the order of `st`; cudaFreeAsync gives them
+// back. What a stream has given back can be trimmed only after a wait for that stream, which
+// costs a short call 13 us: the trim waits, for every stream alive that took from the pool.
+// `own_wait`: the caller waits itself after giving back (its stream may be capturing when
+// another thread trims).
+cudaError_t luz_scratch_alloc(void** p, size_t bytes, cudaStream_t st, bool own_wait = false);
+// Waits for `st`, which is about to be destroyed, and forgets it.
+void luz_scratch_forget(int device, cudaStream_t st);
 // A user of the pool of `device` comes and goes; the last one's leaving empties the pool.
 void luz_scratch_open(int device);
 void luz_scratch_close(int device);
